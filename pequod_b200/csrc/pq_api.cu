@@ -397,13 +397,29 @@ int pq::create_ctx(pq_ctx** out, const pq_model_desc* d, int device, bool helm_o
     const int ntiles_cab_max =
         std::max({cabaret_ctas_bound(ii, jj, L, kMinBand), cabaret_tile_ctas(ii, jj, L), channel_ctas(ii, jj)});
 
-    // Tables.
-    std::vector<double2> tw(M), wsplit(M);
+    // Tables: exp(-2 pi i t / M) and exp(-2 pi i t / N), laid out the way the
+    // row DST reads them (pq_helm.cu: three pass plans, five lane widths).
+    std::vector<double2> tw0(M), ws0(M), tw((size_t)3 * M), wsplit((size_t)5 * M);
     for (int t = 0; t < M; ++t) {
         const long double a = 2.0L * 3.141592653589793238462643383279502884L * (long double)t / (long double)M;
-        tw[t] = make_double2((double)cosl(a), (double)-sinl(a));
+        tw0[t] = make_double2((double)cosl(a), (double)-sinl(a));
         const long double b = 2.0L * 3.141592653589793238462643383279502884L * (long double)t / (long double)N;
-        wsplit[t] = make_double2((double)cosl(b), (double)-sinl(b));
+        ws0[t] = make_double2((double)cosl(b), (double)-sinl(b));
+    }
+    for (int plan = 0; plan < 3; ++plan) {
+        const int most = 8 >> plan;  // largest radix: 8, 4, 2
+        size_t o = (size_t)plan * M;
+        for (int Ns = 1; Ns < M;) {
+            const int rem = M / Ns, R = (most >= 8 && rem >= 8) ? 8 : (most >= 4 && rem >= 4) ? 4 : 2;
+            if (Ns > 1)
+                for (int r = 1; r < R; ++r)
+                    for (int k = 0; k < Ns; ++k) tw[o++] = tw0[(size_t)r * k * (rem / R)];
+            Ns *= R;
+        }
+    }
+    for (int s = 0; s < 5; ++s) {
+        const int V = 2 << s, P = M / V;
+        for (int q = 0; q < P * V; ++q) wsplit[(size_t)s * M + (size_t)(q % V) * P + q / V] = ws0[q];
     }
     std::vector<double> was(N / 2 + 1, 0.0), wmean(n, 0.0);
     for (int k = 1; k <= N / 2; ++k)
@@ -429,18 +445,16 @@ int pq::create_ctx(pq_ctx** out, const pq_model_desc* d, int device, bool helm_o
     };
     const size_t o_fields = take(fb * nfields);
     const size_t o_wind = take(lstride * sizeof(double));
-    const size_t o_tw = take(M * sizeof(double2));
-    const size_t o_ws = take(M * sizeof(double2));
+    const size_t o_tw = take(tw.size() * sizeof(double2));
+    const size_t o_ws = take(wsplit.size() * sizeof(double2));
     const size_t o_was = take(was.size() * sizeof(double));
-    std::vector<float2> tw_f(M), wsplit_f(M);
+    std::vector<float2> tw_f(tw.size()), wsplit_f(wsplit.size());
     std::vector<float> was_f(was.size());
-    for (int t = 0; t < M; ++t) {
-        tw_f[t] = make_float2((float)tw[t].x, (float)tw[t].y);
-        wsplit_f[t] = make_float2((float)wsplit[t].x, (float)wsplit[t].y);
-    }
+    for (size_t t = 0; t < tw.size(); ++t) tw_f[t] = make_float2((float)tw[t].x, (float)tw[t].y);
+    for (size_t t = 0; t < wsplit.size(); ++t) wsplit_f[t] = make_float2((float)wsplit[t].x, (float)wsplit[t].y);
     for (size_t k = 0; k < was.size(); ++k) was_f[k] = (float)was[k];
-    const size_t o_twf = take(M * sizeof(float2));
-    const size_t o_wsf = take(M * sizeof(float2));
+    const size_t o_twf = take(tw_f.size() * sizeof(float2));
+    const size_t o_wsf = take(wsplit_f.size() * sizeof(float2));
     const size_t o_wasf = take(was_f.size() * sizeof(float));
     const size_t o_wm = take(wmean.size() * sizeof(double));
     const size_t o_poff = take(pv.off.size() * sizeof(int));
@@ -525,11 +539,11 @@ int pq::create_ctx(pq_ctx** out, const pq_model_desc* d, int device, bool helm_o
     if (e != cudaSuccess) return fail(c, PQ_ERR_NOMEM, "device allocation failed");
     CK(cudaMemsetAsync(c->arena, 0, off, c->stream));
     char* A = c->arena;
-    CK(cudaMemcpyAsync(A + o_tw, tw.data(), M * sizeof(double2), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(A + o_ws, wsplit.data(), M * sizeof(double2), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(A + o_tw, tw.data(), tw.size() * sizeof(double2), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(A + o_ws, wsplit.data(), wsplit.size() * sizeof(double2), cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(A + o_was, was.data(), was.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(A + o_twf, tw_f.data(), M * sizeof(float2), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(A + o_wsf, wsplit_f.data(), M * sizeof(float2), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(A + o_twf, tw_f.data(), tw_f.size() * sizeof(float2), cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(A + o_wsf, wsplit_f.data(), wsplit_f.size() * sizeof(float2), cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(A + o_wasf, was_f.data(), was_f.size() * sizeof(float), cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(A + o_wm, wmean.data(), wmean.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemcpyAsync(A + o_ww, wwall.data(), wwall.size() * sizeof(double), cudaMemcpyHostToDevice, c->stream));

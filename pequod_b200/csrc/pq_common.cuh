@@ -74,9 +74,9 @@ struct Member {
     double htot;
     double mean_scale;  // 1 / (g_ii_int * g_jj_int)
     // Helmholtz tables (shared between members of the same size)
-    const double2* tw;      // [M]  exp(-2 pi i t / M)
+    const double2* tw;      // [3][M] pass twiddles, by pass plan (pq_helm.cu)
     const double* was;      // [N/2] 2 sin(k pi / N), index k (0 unused)
-    const double2* wsplit;  // [M]  exp(-2 pi i q / N)
+    const double2* wsplit;  // [5][M] exp(-2 pi i q / N), by values per lane
     const double* wmean;    // [n]  2 * sum_i sin(i k pi / N), index k-1
     const float2* tw_f;     // FP32 copies of tw, wsplit, was (mixed path)
     const float2* wsplit_f;

@@ -5,7 +5,7 @@
 // solve along j with precomputed reciprocal pivots (ge_local, :1028-1059),
 // and the inverse DST (helm, :614-769).  Here that is three kernels:
 //
-//   k_dst_rows<FWD>  one CTA per interior row j: load (optionally apply the
+//   k_dst (forward)  one CTA per interior row j: load (optionally apply the
 //                    CABARET predictor + beta step and the z_to_modes
 //                    projection), scale by 0.5/(ii-1), DST every mode row in
 //                    shared memory, write the spectral rows.
@@ -17,7 +17,7 @@
 //                    warp scan of the affine chunk maps, fix-up sweep).  The
 //                    same CTA accumulates the domain mean of the solution in
 //                    spectral space; the last CTA of a member finishes psiC.
-//   k_dst_rows<INV>  one CTA per row j: inverse DST of every mode row, then
+//   k_dst (inverse)  one CTA per row j: inverse DST of every mode row, then
 //                    the mass-corrected back-projection (modes_to_z_btcu,
 //                    qg3p_diagnostics.F90:615-635) straight into psi.
 //
@@ -43,16 +43,16 @@ constexpr int TRI_THREADS = 256;
 // Row DSTs: one group of P lanes per (row, mode) unit.
 //
 // The complex FFT of length M = N/2 is a Stockham FFT in which every lane of
-// a group owns V = M / P values for the whole transform: the pre-twiddle
-// computes a lane's first-pass inputs straight into registers, each radix-8
-// (then 4 or 2) pass is a set of V/R in-register butterflies, and values cross
-// lanes only through the unit's shared-memory row between passes (under
-// __syncwarp, never a block barrier).  The real-FFT split and the prefix sum
+// a group owns V = M / P values per pass: the row is loaded as node pairs and
+// stored pre-twiddled (put_pair), each radix-8 (then 4 or 2) pass is a set of
+// V/R in-register butterflies, and values cross lanes only through the unit's
+// shared-memory row between passes (under __syncwarp or the unit's named
+// barrier, never a block barrier).  The real-FFT split and the prefix sum
 // of the odd outputs run on V contiguous wavenumbers per lane with one
 // segmented warp scan.  V = 8 up to M = 256 (P = M/8 lanes), then 16, 32.
 //
-// Unit buffer (U scalars per unit): plain real row x[k] (input), padded
-// complex rows (Stockham passes, index t -> t + t/8), padded real output row
+// Unit buffer (U scalars per unit): padded complex rows (the pre-twiddled
+// sequence and the Stockham passes, index t -> t + t/8), padded real output row
 // (index k -> k + 2*(k/16), so that the pair stores of the split are
 // bank-conflict free).
 
@@ -64,6 +64,27 @@ template <typename T2> __device__ __forceinline__ T2 c_mi(T2 a) {  // a * (-i)
     r.x = a.y;
     r.y = -a.x;
     return r;
+}
+
+// The FP32 transform's products and sums are written out as the multiply-adds
+// they are, so that every instance (lanes, values per lane, one member or
+// many) rounds alike whatever the compiler would contract around them: a
+// mixed run's trajectory does not depend on the geometry of its launches.
+// FP64 leaves the contraction to the compiler, which folds a twiddle product
+// into the butterfly's sums (two operations fewer, one rounding fewer).
+__device__ __forceinline__ double mad(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float mad(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double2 tw_mul(double2 a, double2 w) { return cmul(a, w); }
+__device__ __forceinline__ float2 tw_mul(float2 a, float2 w) {
+    return make_float2(__fmaf_rn(a.x, w.x, -__fmul_rn(a.y, w.y)), __fmaf_rn(a.x, w.y, __fmul_rn(a.y, w.x)));
+}
+// e + w o
+__device__ __forceinline__ double2 split_sum(double2 e, double2 w, double2 o) {
+    return make_double2(e.x + (w.x * o.x - w.y * o.y), e.y + (w.x * o.y + w.y * o.x));
+}
+__device__ __forceinline__ float2 split_sum(float2 e, float2 w, float2 o) {
+    const float2 t = tw_mul(o, w);
+    return make_float2(__fadd_rn(e.x, t.x), __fadd_rn(e.y, __fmaf_rn(w.x, o.y, __fmul_rn(w.y, o.x))));
 }
 
 // In-register forward DFT of R points (R = 2, 4, 8), natural order.
@@ -84,24 +105,23 @@ template <int R, typename T2> __device__ __forceinline__ void dft_reg(T2* v) {
         const T2 e0 = cadd(v[0], v[4]), e1 = csub(v[0], v[4]), e2 = cadd(v[2], v[6]), e3 = c_mi(csub(v[2], v[6]));
         const T2 E0 = cadd(e0, e2), E1 = cadd(e1, e3), E2 = csub(e0, e2), E3 = csub(e1, e3);
         const T2 o0 = cadd(v[1], v[5]), o1 = csub(v[1], v[5]), o2 = cadd(v[3], v[7]), o3 = c_mi(csub(v[3], v[7]));
-        T2 O0 = cadd(o0, o2), O1 = cadd(o1, o3), O2 = csub(o0, o2), O3 = csub(o1, o3);
+        const T2 O0 = cadd(o0, o2), O1 = cadd(o1, o3), O3 = csub(o1, o3);
+        T2 O2 = csub(o0, o2);
         // W8^1 = (1 - i)/sqrt2, W8^2 = -i, W8^3 = (-1 - i)/sqrt2
-        T2 t;
-        t.x = c8 * (O1.x + O1.y);
-        t.y = c8 * (O1.y - O1.x);
-        O1 = t;
+        const T s1x = O1.x + O1.y, s1y = O1.y - O1.x, s3x = O3.y - O3.x, s3y = -(O3.x + O3.y);
         O2 = c_mi(O2);
-        t.x = c8 * (O3.y - O3.x);
-        t.y = -c8 * (O3.x + O3.y);
-        O3 = t;
         v[0] = cadd(E0, O0);
-        v[1] = cadd(E1, O1);
+        v[1].x = mad(c8, s1x, E1.x);
+        v[1].y = mad(c8, s1y, E1.y);
         v[2] = cadd(E2, O2);
-        v[3] = cadd(E3, O3);
+        v[3].x = mad(c8, s3x, E3.x);
+        v[3].y = mad(c8, s3y, E3.y);
         v[4] = csub(E0, O0);
-        v[5] = csub(E1, O1);
+        v[5].x = mad(-c8, s1x, E1.x);
+        v[5].y = mad(-c8, s1y, E1.y);
         v[6] = csub(E2, O2);
-        v[7] = csub(E3, O3);
+        v[7].x = mad(-c8, s3x, E3.x);
+        v[7].y = mad(-c8, s3y, E3.y);
     }
 }
 
@@ -114,29 +134,41 @@ __device__ __forceinline__ void unit_sync(int P, int uid) {
         asm volatile("bar.sync %0, %1;\n" ::"r"(1 + uid), "r"(P) : "memory");
 }
 
+// Twiddle tables (built by the host, Member::tw / wsplit, FP32 copies beside):
+//   tw      three sections of M entries, one per pass plan (radix 8, then a 4
+//           or 2, for V >= 8; radix 4, then a 2, for V = 4; radix 2 for V = 2).
+//           A plan's passes follow one another (the first needs none); the
+//           pass on sub-transforms of length Ns holds exp(-2 pi i r k / (Ns R))
+//           at (r - 1) Ns + k, so lanes with consecutive k read consecutive
+//           entries.
+//   wsplit  five sections of M entries, V = 2, 4, 8, 16, 32: the split weight
+//           of wavenumber q = p V + e at e P + p, again one line per warp.
+// (Both were indexed by the angle before: every 16-byte load of the split
+// touched 32 lines and those of a pass up to 28, about 40 % of the kernel's
+// L1 cycles at 1025 nodes.)
+template <int V> __host__ __device__ constexpr int dst_plan() { return V >= 8 ? 0 : V == 4 ? 1 : 2; }
+template <int V> __host__ __device__ constexpr int dst_split_section() { return V == 2 ? 0 : V == 4 ? 1 : V == 8 ? 2 : V == 16 ? 3 : 4; }
+
 // One radix-R Stockham pass over the unit's M values (Ns = length of the
 // sub-transforms already done).  Lane p owns butterflies j = p + P*b; its
-// values v[b*R + r] are the butterfly inputs j + r*(M/R).  With `load` false
-// the inputs are already in registers (first pass).  Output is stored to the
-// unit's padded complex row.
+// values v[b*R + r] are the butterfly inputs j + r*(M/R), read from and stored
+// to the unit's padded complex row.  tw: this pass's table (unused at Ns = 1).
 template <int V, int R, typename T2>
-__device__ __forceinline__ void fft_pass(T2 (&v)[V], T2* z, int p, int P, int uid, int M, int logM, int Ns,
-                                         int logNs, const T2* __restrict__ tw, bool load) {
+__device__ __forceinline__ void fft_pass(T2* z, int p, int P, int uid, int M, int Ns, int logNs,
+                                         const T2* __restrict__ tw) {
     constexpr int logR = (R == 8) ? 3 : (R == 4) ? 2 : 1;
     const int MR = M >> logR;
-    if (load) {
+    T2 v[V];
 #pragma unroll
-        for (int b = 0; b < V / R; ++b)
+    for (int b = 0; b < V / R; ++b)
 #pragma unroll
-            for (int r = 0; r < R; ++r) v[b * R + r] = z[cpad(p + P * b + r * MR)];
-    }
-    const int lst = logM - logR - logNs;  // log2(M / (Ns R))
+        for (int r = 0; r < R; ++r) v[b * R + r] = z[cpad(p + P * b + r * MR)];
 #pragma unroll
     for (int b = 0; b < V / R; ++b) {
-        const int j = p + P * b, k = j & (Ns - 1);
-        if (k) {
+        const int k = (p + P * b) & (Ns - 1);
+        if (Ns > 1) {
 #pragma unroll
-            for (int r = 1; r < R; ++r) v[b * R + r] = cmul(v[b * R + r], __ldg(&tw[(r * k) << lst]));
+            for (int r = 1; r < R; ++r) v[b * R + r] = tw_mul(v[b * R + r], __ldg(&tw[((r - 1) << logNs) + k]));
         }
         dft_reg<R>(&v[b * R]);
     }
@@ -151,68 +183,85 @@ __device__ __forceinline__ void fft_pass(T2 (&v)[V], T2* z, int p, int P, int ui
     unit_sync(P, uid);
 }
 
-// DST-I (FFTPACK sint convention, qg3p_helmholtz.F90:1370-1426) of the real
-// row held in the unit buffer (x_k at buf[k], k = 1..N-1), output X_k at
-// buf[xpad(k)], k = 1..N-1.  Every lane of the unit must call this; uid
+// The pre-twiddled sequence of a row (sint1, qg3p_helmholtz.F90:1404-1413):
+// c_k = (x_k - x_{N-k}) + 2 sin(k pi / N) (x_k + x_{N-k}), c_0 = 0, stored
+// packed as c_{2t} + i c_{2t+1} in the unit's padded complex row.  Pair t of
+// nodes (t, N - t), t = 1..N/2-1, gives c_t and c_{N-t}; pair 0 stands for
+// the middle node N/2 (xb = xa) and c_0.
+__device__ __forceinline__ int cidx(int k) { return 2 * cpad(k >> 1) + (k & 1); }
+template <typename T>
+__device__ __forceinline__ void put_pair(T* buf, int t, int N, T xa, T xb, const T* __restrict__ was) {
+    const int k = t ? t : N >> 1;
+    const T w = __ldg(&was[k]);
+    buf[cidx(k)] = mad(w, xa + xb, xa - xb);
+    if (t)
+        buf[cidx(N - k)] = mad(w, xa + xb, xb - xa);
+    else
+        buf[0] = (T)0;
+}
+// A unit's own row, straight from global memory (fetch(k) is x_k): V pairs per lane,
+// at most eight of them in flight.
+template <int V, typename T, typename F>
+__device__ __forceinline__ void stage_unit(T* buf, int p, int P, int N, const T* __restrict__ was, F fetch) {
+    constexpr int B = V < 8 ? V : 8;
+#pragma unroll
+    for (int e0 = 0; e0 < V; e0 += B) {
+        T xa[B], xb[B];
+#pragma unroll
+        for (int e = 0; e < B; ++e) {
+            const int t = p + P * (e0 + e), k = t ? t : N >> 1;
+            xa[e] = fetch(k);
+            xb[e] = fetch(N - k);
+        }
+#pragma unroll
+        for (int e = 0; e < B; ++e) put_pair(buf, p + P * (e0 + e), N, xa[e], xb[e], was);
+    }
+}
+
+// DST-I (FFTPACK sint convention, qg3p_helmholtz.F90:1370-1426) of the row
+// whose pre-twiddled sequence the unit buffer holds (put_pair), output X_k
+// at buf[xpad(k)], k = 1..N-1.  Every lane of the unit must call this; uid
 // names the unit's barrier, utot is P/32 scalars of scratch for units wider
 // than a warp.
-template <int V, typename T>
-__device__ __forceinline__ void dst_unit(T* buf, int p, int P, int uid, T* utot, int N, int M, int logM,
+template <int V, int M, int Ns, typename T2>
+__device__ __forceinline__ void fft_passes(T2* z, int p, int uid, const T2* __restrict__ tw) {
+    if constexpr (Ns < M) {
+        constexpr int rem = M / Ns, R = (V >= 8 && rem >= 8) ? 8 : (V >= 4 && rem >= 4) ? 4 : 2;
+        constexpr int logNs = Ns == 1 ? 0 : 31 - __builtin_clz((unsigned)Ns);
+        fft_pass<V, R>(z, p, M / V, uid, M, Ns, logNs, tw);
+        fft_passes<V, M, Ns * R>(z, p, uid, tw + (Ns > 1 ? (R - 1) * Ns : 0));
+    }
+}
+template <int V, int PC, typename T>
+__device__ __forceinline__ void dst_unit(T* buf, int p, int P, int uid, T* utot, int N, int M,
                                          const typename Cplx<T>::type* __restrict__ tw,
-                                         const typename Cplx<T>::type* __restrict__ wsp,
-                                         const T* __restrict__ was) {
+                                         const typename Cplx<T>::type* __restrict__ wsp) {
     using T2 = typename Cplx<T>::type;
     constexpr int R0 = V >= 8 ? 8 : V;
-    T2 v[V];
-    // Pre-twiddle (sint1, :1404-1413) into the first pass's inputs:
-    // c_k = (x_k - x_{N-k}) + 2 sin(k pi / N) (x_k + x_{N-k}), c_0 = 0,
-    // packed c_{2t} + i c_{2t+1}.
-    {
-        const int MR0 = M / R0;
-#pragma unroll
-        for (int b = 0; b < V / R0; ++b)
-#pragma unroll
-            for (int r = 0; r < R0; ++r) {
-                const int t = p + P * b + r * MR0;
-                const int k = 2 * t;
-                const T2 xa = *reinterpret_cast<const T2*>(buf + k);  // x_k, x_{k+1}
-                const T xb0 = buf[N - k], xb1 = buf[N - k - 1];
-                const bool lo = 2 * k < N;  // then k + 1 <= N/2 too
-                const T w0 = __ldg(&was[lo ? k : N - k]), w1 = __ldg(&was[lo ? k + 1 : N - k - 1]);
-                const T c0 = (t == 0) ? (T)0 : (xa.x - xb0) + w0 * (xa.x + xb0);
-                const T c1 = (xa.y - xb1) + w1 * (xa.y + xb1);
-                v[b * R0 + r].x = c0;
-                v[b * R0 + r].y = c1;
-            }
-    }
     T2* z = reinterpret_cast<T2*>(buf);
-    {
+    tw += dst_plan<V>() * M;
+    wsp += dst_split_section<V>() * M;
+    if constexpr (PC > 0) {
+        fft_passes<V, V * PC, 1>(z, p, uid, tw);
+    } else {
         int Ns = 1, logNs = 0;
-        bool first = true;
         while (Ns < M) {
             const int rem = M >> logNs;
-            if constexpr (V >= 8) {
-                if (rem >= 8) {
-                    fft_pass<V, 8>(v, z, p, P, uid, M, logM, Ns, logNs, tw, !first);
-                    Ns <<= 3;
-                    logNs += 3;
-                    first = false;
-                    continue;
-                }
+            int done = 2, ldone = 1;
+            if (V >= 8 && rem >= 8) {
+                if constexpr (V >= 8) fft_pass<V, 8>(z, p, P, uid, M, Ns, logNs, tw);
+                done = 8;
+                ldone = 3;
+            } else if (R0 >= 4 && rem >= 4) {
+                if constexpr (R0 >= 4) fft_pass<V, 4>(z, p, P, uid, M, Ns, logNs, tw);
+                done = 4;
+                ldone = 2;
+            } else {
+                fft_pass<V, 2>(z, p, P, uid, M, Ns, logNs, tw);
             }
-            if constexpr (V >= 4) {
-                if (rem >= 4) {
-                    fft_pass<V, 4>(v, z, p, P, uid, M, logM, Ns, logNs, tw, !first);
-                    Ns <<= 2;
-                    logNs += 2;
-                    first = false;
-                    continue;
-                }
-            }
-            fft_pass<V, 2>(v, z, p, P, uid, M, logM, Ns, logNs, tw, !first);
-            Ns <<= 1;
-            logNs += 1;
-            first = false;
+            if (Ns > 1) tw += (done - 1) * Ns;
+            Ns *= done;
+            logNs += ldone;
         }
     }
     // Real-FFT split on V contiguous wavenumbers q = p*V + e:
@@ -225,14 +274,14 @@ __device__ __forceinline__ void dst_unit(T* buf, int p, int P, int uid, T* utot,
         const int q = p * V + e;
         const T2 zq = z[cpad(q)];
         const T2 zr = z[cpad((M - q) & (M - 1))];
-        const T ex = (T)0.5 * (zq.x + zr.x), ey = (T)0.5 * (zq.y - zr.y);
         const T dx = zq.x - zr.x, dy = zq.y + zr.y;
-        T2 O;
+        T2 E, O;
+        E.x = (T)0.5 * (zq.x + zr.x);
+        E.y = (T)0.5 * (zq.y - zr.y);
         O.x = (T)0.5 * dy;
         O.y = (T)-0.5 * dx;
-        const T2 w = __ldg(&wsp[q]);
-        const T cx = ex + (w.x * O.x - w.y * O.y);
-        const T cy = ey + (w.x * O.y + w.y * O.x);
+        const T2 C = split_sum(E, __ldg(&wsp[e * P + p]), O);
+        const T cx = C.x, cy = C.y;
         Xe[e] = (q == 0) ? (T)0 : -cy;
         run += (q == 0) ? (T)0.5 * cx : cx;
         Xo[e] = run;
@@ -251,9 +300,10 @@ __device__ __forceinline__ void dst_unit(T* buf, int p, int P, int uid, T* utot,
         T add = (T)0;
         for (int w = 0; w < (p >> 5); ++w) add += utot[w];
         incl += add;
+    } else {
+        unit_sync(P, uid);
     }
     const T excl = incl - run;
-    unit_sync(P, uid);
 #pragma unroll
     for (int e = 0; e < V; ++e) {
         const int q = p * V + e;
@@ -293,43 +343,54 @@ __device__ __forceinline__ void cp16(void* dst, const void* src, bool ok) {
     const unsigned sa = (unsigned)__cvta_generic_to_shared(dst);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sa), "l"(src), "r"(ok ? 16 : 0) : "memory");
 }
-__device__ __forceinline__ void cp8z(double* dst, const double* src, bool ok) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(sa), "l"(src), "r"(ok ? 8 : 0) : "memory");
-}
 __device__ __forceinline__ void cp_commit_wait_all() {
     asm volatile("cp.async.commit_group;\n" ::: "memory");
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-}
-
-__device__ __forceinline__ void cp4z(void* dst, const void* src, bool ok) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(sa), "l"(src), "r"(ok ? 4 : 0) : "memory");
 }
 
 // Row DST kernel.  A CTA holds R rows x L modes = L*R units of P lanes,
 // ordered mode-major (unit (m, r) at index m*R + r), so that every warp's
 // units share one mode.
 //
-// Forward (EPI_SPEC, interior rows 1..jj-2): the raw layer rows are copied
-// asynchronously into shared memory (16-byte copies: node k of a row and
-// entry k of the buffer have the same alignment), projected onto the modes
-// (z_to_modes) and scaled by 0.5/(ii-1); PRO_STEP instead computes the
-// CABARET predictor + beta update per node in registers.  Each unit then
-// transforms its row and writes spec(m, j, k-1) = X_k.
+// Forward (EPI_SPEC, interior rows 1..jj-2): a thread loads the layer values
+// of a node pair (k, N - k) straight from global memory, projects both onto
+// the modes (z_to_modes, scaled by 0.5/(ii-1); PRO_STEP first applies the
+// CABARET predictor + beta update, PRO_PLAIN only scales) and stores the
+// pair's two pre-twiddled values of every mode.  Each unit then transforms
+// its row and writes spec(m, j, k-1) = X_k.
 //
-// Inverse (EPI_HELM / EPI_PV, rows 0..jj-1): the solved spectral rows are
-// copied in (spec offset k-1 -> buffer entry k), transformed, and written
-// out; for EPI_PV the correction rows corr_m (m >= 1) are prefetched into
-// shared memory before the transform and the mass-corrected back-projection
-// writes psi.
+// Inverse (EPI_HELM / EPI_PV, rows 0..jj-1): each unit loads the pairs of its
+// solved spectral row (zero on the boundary rows), transforms them, and the
+// row is written out; for EPI_PV the correction rows corr_m (m >= 1) are
+// copied into shared memory during the transform and the mass-corrected
+// back-projection writes psi.
+//
+// What bounds it: L1 / shared-memory cycles and the latency of a CTA's chain
+// (1.7 waves at 1025 nodes).  Pre-twiddling in registers, instead of staging
+// the row (cp.async), projecting it in place and reading it twice more, takes
+// five passes over the shared-memory row down to two; with the tables read
+// line by line, FP32 units at their own width and compile-time geometries:
+// 1025^2 x 3 forward 45.7 -> 29.1 us FP64, 33.4 -> 24.8 mixed, inverse 41.1 ->
+// 27.6 and 36.7 -> 26.7; 2049^2 x 5 forward 271 -> 169 and 236 -> 144, inverse
+// 291 -> 177 and 257 -> 156 (there two CTAs per SM instead of one).
 //
 // S is the storage type of the state and spectral fields.  S = float is the
 // mixed form: the layer fields and the baroclinic spectral rows are FP32 and
 // transformed in FP32, while the barotropic mode (m = 0) is kept in FP64
 // end to end (spec64), as are the projection, the back-projection and psi.
+// Scalars of shared memory (in doubles) the L*R unit buffers take: FP64, or
+// for the mixed form FP64 for mode 0 and FP32 for the others.
+__host__ __device__ inline size_t dst_units_len(int L, int R, int N, bool mixed) {
+    const size_t U = dst_unit_len(N);
+    return mixed ? R * U + (((size_t)(L - 1) * R * U + 3) / 4) * 2 : (size_t)L * R * U;
+}
+
 // The row-DST kernel's body; k_dst and k_dst_capped below are its kernels.
-template <typename S, int V, int PRO, int EPI>
+//
+// PC > 0: the lanes per unit P at compile time (the default geometries of the
+// grids up to 2049 nodes), hence N, M and the pitch: every index of the
+// transform is then a lane's base plus an immediate.
+template <typename S, int V, int PC, int PRO, int EPI>
 __device__ __forceinline__ void dst_body(const Member* __restrict__ mems, const int* __restrict__ prefix, int nmem,
                                          int row_offset, int c, int corr_smem, int psic_here, const Member& one,
                                          int use_one, int gemm_bc) {
@@ -342,199 +403,95 @@ __device__ __forceinline__ void dst_body(const Member* __restrict__ mems, const 
     int local;
     cta_member(Mb, one, use_one, mems, prefix, nmem, blockIdx.x, &local);
     __syncthreads();
-    const int L = Mb.L, N = Mb.N, M = Mb.M, logM = Mb.logM, n = Mb.n, ii = Mb.ii, jj = Mb.jj, pitch = Mb.pitch;
+    const int L = Mb.L, jj = Mb.jj;
+    const int P = PC ? PC : Mb.M / V;
+    const int M = P * V, N = 2 * M, n = N - 1, ii = N + 1, pitch = (ii + 31) & ~31;
     const long long ls = Mb.lstride;
-    const int P = M / V;
     const int R = dst_rows_per_cta(P, c);
     const int U = dst_unit_len(N);
     const int j0 = row_offset + local * R;                 // first row of this CTA
     // one past the last row; a channel periodic in j transforms every row
     const int jend = (EPI == EPI_SPEC && !Mb.periodic) ? jj - 1 : jj;
     const int nthr = blockDim.x;
-    double* extra = sm + (size_t)L * R * U;                 // EPI_PV: corr rows [R][L-1][pitch];
-                                                            // mixed forward: staged rows [R][L][N] (FP32)
+    double* extra = sm + dst_units_len(L, R, N, MX);        // EPI_PV: corr rows [R][L-1][pitch]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarp = nthr >> 5;
-    auto ubuf = [&](int m, int r) { return sm + (size_t)(m * R + r) * U; };
-    // Unit (m, r) buffers hold FP64 values, except the baroclinic ones of the mixed form.
+    // Unit (m, r) buffers: FP64 values, except the baroclinic ones of the mixed form.
     auto fp64_mode = [&](int m) { return !MX || m == 0; };
-    auto put = [&](int m, int r, int k, double v) {
-        if (fp64_mode(m))
-            ubuf(m, r)[k] = v;
-        else
-            reinterpret_cast<float*>(ubuf(m, r))[k] = (float)v;
-    };
-    auto get = [&](int m, int r, int k) -> double {
-        return fp64_mode(m) ? ubuf(m, r)[k] : (double)reinterpret_cast<const float*>(ubuf(m, r))[k];
-    };
+    auto ubuf = [&](int m, int r) { return sm + (size_t)(m * R + r) * U; };  // FP64 modes
+    auto ubuf32 = [&](int m, int r) { return reinterpret_cast<float*>(sm + (size_t)R * U) + (size_t)((m - 1) * R + r) * U; };
+    auto get = [&](int m, int r, int k) -> double { return fp64_mode(m) ? ubuf(m, r)[k] : (double)ubuf32(m, r)[k]; };
+    // This thread's unit: mode um of row ju.
+    const int u = threadIdx.x / P, p = threadIdx.x & (P - 1);
+    const int um = u / R, ur = u - um * R;
+    const int ju = j0 + ur;
+    const bool interior = (Mb.periodic || (ju >= 1 && ju <= jj - 2)) && ju < jend;
 
     // ---------------- stage the rows --------------------------------------
     if (EPI == EPI_SPEC) {
         const double cff = 0.5 / (double)(ii - 1);
-        if (PRO != PRO_STEP) {
+        // The pair's values xa (node k), xb (node N - k) of mode m, row r.
+        auto put = [&](int m, int r, int t, double xa, double xb) {
+            if (fp64_mode(m)) {
+                put_pair(ubuf(m, r), t, N, xa, xb, Mb.was);
+            } else if (gemm_bc) {
+                // the projected node row itself, for the tensor-core DST
+                if (j0 + r < jend) {
+                    float* g = reinterpret_cast<float*>(Mb.gbuf) + m * ls + (long long)(j0 + r) * pitch - 1;
+                    const int k = t ? t : N >> 1;
+                    g[k] = (float)xa;
+                    if (t) g[N - k] = (float)xb;
+                }
+            } else {
+                put_pair(ubuf32(m, r), t, N, (float)xa, (float)xb, Mb.was_f);
+            }
+        };
+        if constexpr (PRO == PRO_PLAIN) {
             // The stand-alone helm input (helm_io) is FP64 in either form.
-            using ST = std::conditional_t<PRO == PRO_PLAIN, double, S>;
-            const ST* src = reinterpret_cast<const ST*>(PRO == PRO_PLAIN ? Mb.helm_io : Mb.zeta);
-            // Layer l of row j0 + r: FP64 into unit (l, r) (projected in place
-            // below), FP32 into the staging rows; one warp per row.
-            constexpr int PER16 = 16 / sizeof(ST);
-            for (int rl = warp; rl < R * L; rl += nwarp) {
-                const int r = rl / L, l = rl - r * L;
-                const int j = j0 + r;
-                const bool ok = j < jend;
-                const ST* g = src + l * ls + (long long)(ok ? j : 1) * pitch;
-                ST* d = MX ? reinterpret_cast<ST*>(extra) + (size_t)rl * N : reinterpret_cast<ST*>(ubuf(l, r));
-                for (int q = lane; q < N / PER16; q += 32) cp16(d + PER16 * q, g + PER16 * q, ok);
+            const double* src = reinterpret_cast<const double*>(Mb.helm_io) + um * ls +
+                                (long long)(ju < jend ? ju : jend - 1) * pitch;
+            if (fp64_mode(um)) {
+                stage_unit<V>(ubuf(um, ur), p, P, N, Mb.was, [&](int k) { return cff * __ldg(src + k); });
+            } else if (gemm_bc) {
+                for (int t = p; t < M; t += P) put(um, ur, t, cff * __ldg(src + (t ? t : M)), cff * __ldg(src + N - t - (t ? 0 : M)));
+            } else {
+                stage_unit<V>(ubuf32(um, ur), p, P, N, Mb.was_f, [&](int k) { return (float)(cff * __ldg(src + k)); });
             }
-            cp_commit_wait_all();
-            __syncthreads();
-            // Node k of the L layer rows -> node k of the L mode rows (in
-            // place for FP64: a node's values are read before they are written).
-            // z_to_modes with an exact layer count up to five: loops unrolled to
-            // L, z2m in registers (as the back-projection below).
-            auto exact = [&](auto lc) {
-                constexpr int LC = decltype(lc)::value;
-                double zm[LC][LC];
-#pragma unroll
-                for (int m = 0; m < LC; ++m)
-#pragma unroll
-                    for (int l = 0; l < LC; ++l) zm[m][l] = Mb.z2m[m * PQ_MAXL + l];
-                for (int r = 0; r < R; ++r)
-                    for (int k = threadIdx.x; k < N; k += nthr) {
-                        double z[LC];
-#pragma unroll
-                        for (int l = 0; l < LC; ++l)
-                            z[l] = MX ? (double)reinterpret_cast<const ST*>(extra)[(size_t)(r * LC + l) * N + k]
-                                      : ubuf(l, r)[k];
-#pragma unroll
-                        for (int m = 0; m < LC; ++m) {
-                            // z_to_modes, qg3p_diagnostics.F90:545-549
-                            double sacc = 0.0;
-#pragma unroll
-                            for (int l = 0; l < LC; ++l) sacc += zm[m][l] * z[l];
-                            put(m, r, k, cff * sacc);
-                        }
-                    }
-            };
-            bool done = false;
-            if constexpr (PRO == PRO_MODAL) {
-                done = true;
-                switch (L) {
-                    case 1: exact(std::integral_constant<int, 1>{}); break;
-                    case 2: exact(std::integral_constant<int, 2>{}); break;
-                    case 3: exact(std::integral_constant<int, 3>{}); break;
-                    case 4: exact(std::integral_constant<int, 4>{}); break;
-                    case 5: exact(std::integral_constant<int, 5>{}); break;
-                    default: done = false;
-                }
-            }
-            if (!done)
-            for (int r = 0; r < R; ++r)
-                for (int k = threadIdx.x; k < N; k += nthr) {
-                    double z[PQ_MAXL];
-#pragma unroll
-                    for (int l = 0; l < PQ_MAXL; ++l)
-                        if (l < L)
-                            z[l] = MX ? (double)reinterpret_cast<const ST*>(extra)[(size_t)(r * L + l) * N + k]
-                                      : ubuf(l, r)[k];
-                    if constexpr (PRO == PRO_PLAIN) {
-#pragma unroll
-                        for (int m = 0; m < PQ_MAXL; ++m)
-                            if (m < L) put(m, r, k, cff * z[m]);
-                    } else {
-#pragma unroll 1
-                        for (int m = 0; m < L; ++m) {
-                            // z_to_modes, qg3p_diagnostics.F90:545-549
-                            double sacc = 0.0;
-#pragma unroll
-                            for (int l = 0; l < PQ_MAXL; ++l)
-                                if (l < L) sacc += Mb.z2m[m * PQ_MAXL + l] * z[l];
-                            put(m, r, k, cff * sacc);
-                        }
-                    }
-                }
         } else {
             const double dt = Mb.sc->dt, ta = Mb.sc->tweight_a;
+            const S* __restrict__ zin = reinterpret_cast<const S*>(Mb.zeta);
             const S* __restrict__ zo = reinterpret_cast<const S*>(Mb.zeta_old[Mb.cur]);
             const S* __restrict__ rs = reinterpret_cast<const S*>(Mb.res);
             const S* __restrict__ rbo = reinterpret_cast<const S*>(Mb.res_beta_other);
             S* __restrict__ rb = reinterpret_cast<S*>(Mb.res_beta);
             const S* __restrict__ ui = reinterpret_cast<const S*>(Mb.ui);
             S* __restrict__ zp = reinterpret_cast<S*>(Mb.zeta);
-            // Exact layer counts up to five: loops unrolled to L, beta and
-            // z2m in registers (as the modal prologue); the same arithmetic.
-            auto exact = [&](auto lc) {
+            // Layer counts up to five run with the loops unrolled to the exact
+            // count and z2m (and beta) in registers, larger ones under predicates.
+            auto rows = [&](auto lc, auto exact) {
                 constexpr int LC = decltype(lc)::value;
-                double zm[LC][LC], bt[LC];
+                constexpr bool EX = decltype(exact)::value;
+                // Node pairs a thread loads before it uses any of them.
+                constexpr int UN = PRO == PRO_STEP ? 1 : LC <= 2 ? 3 : LC == 3 ? 2 : 1;
+                // z2m in registers up to three layers, else read from shared memory.
+                constexpr bool ZR = EX && LC <= 3;
+                constexpr int LZ = ZR ? LC : 1;
+                double zm[LZ][LZ];
+                if constexpr (ZR) {
 #pragma unroll
-                for (int m = 0; m < LC; ++m) {
-                    bt[m] = Mb.beta[m];
+                    for (int m = 0; m < LC; ++m)
 #pragma unroll
-                    for (int l = 0; l < LC; ++l) zm[m][l] = Mb.z2m[m * PQ_MAXL + l];
+                        for (int l = 0; l < LC; ++l) zm[m][l] = Mb.z2m[m * PQ_MAXL + l];
                 }
-                for (int r = 0; r < R; ++r) {
-                    const int j = j0 + r;
-                    const bool ok = j < jend;
-                    for (int k = 1 + threadIdx.x; k <= n; k += nthr) {
-                        const long long o = (long long)j * pitch + k;
-                        double a0[LC], a1[LC], a2[LC], a3[LC], a4[LC];
-#pragma unroll
-                        for (int l = 0; l < LC; ++l) {
-                            if (ok) {
-                                const long long ol = o + l * ls;
-                                a0[l] = zo[ol];
-                                a1[l] = rs[ol];
-                                a2[l] = ui[ol];
-                                a3[l] = ui[ol + 1];
-                                a4[l] = rbo[ol];
-                            }
-                        }
-                        double z[LC];
-#pragma unroll
-                        for (int l = 0; l < LC; ++l) {
-                            double zz = 0.0;
-                            if (ok) {
-                                const long long ol = o + l * ls;
-                                // cabaret_predictor, qg3p_aux.F90:1012-1018
-                                zz = a0[l] + 0.5 * dt * a1[l];
-                                // cabaret_beta, qg3p_aux.F90:1051-1059
-                                const double rbn = dt * (0.5 * (a3[l] + a2[l]) * bt[l]);
-                                zz = zz + (1.0 + ta) * rbn - ta * a4[l];
-                                rb[ol] = (S)rbn;
-                                zp[ol] = (S)zz;
-                                if (MX) zz = (double)(S)zz;  // the stored (FP32) value
-                            }
-                            z[l] = zz;
-                        }
-#pragma unroll
-                        for (int m = 0; m < LC; ++m) {
-                            double sacc = 0.0;
-#pragma unroll
-                            for (int l = 0; l < LC; ++l) sacc += zm[m][l] * z[l];
-                            put(m, r, k, cff * sacc);
-                        }
-                    }
-                }
-            };
-            bool done = true;
-            switch (L) {
-                case 1: exact(std::integral_constant<int, 1>{}); break;
-                case 2: exact(std::integral_constant<int, 2>{}); break;
-                case 3: exact(std::integral_constant<int, 3>{}); break;
-                case 4: exact(std::integral_constant<int, 4>{}); break;
-                case 5: exact(std::integral_constant<int, 5>{}); break;
-                default: done = false;
-            }
-            if (!done)
-            for (int r = 0; r < R; ++r) {
-                const int j = j0 + r;
-                const bool ok = j < jend;
-                for (int k = 1 + threadIdx.x; k <= n; k += nthr) {
+                auto has = [&](int l) { return EX || l < L; };
+                // cabaret_predictor (qg3p_aux.F90:1012-1018) and cabaret_beta
+                // (:1051-1059) at node k of row j: every load first, then the
+                // arithmetic and the stores of res_beta and zeta.
+                auto step_node = [&](int j, int k, bool ok, double (&z)[LC]) {
                     const long long o = (long long)j * pitch + k;
-                    double a0[PQ_MAXL], a1[PQ_MAXL], a2[PQ_MAXL], a3[PQ_MAXL], a4[PQ_MAXL];
-                    // All loads of the node first, then the arithmetic and stores.
+                    double a0[LC], a1[LC], a2[LC], a3[LC], a4[LC];
 #pragma unroll
-                    for (int l = 0; l < PQ_MAXL; ++l) {
-                        if (l < L && ok) {
+                    for (int l = 0; l < LC; ++l) {
+                        if (has(l) && ok) {
                             const long long ol = o + l * ls;
                             a0[l] = zo[ol];
                             a1[l] = rs[ol];
@@ -543,71 +500,133 @@ __device__ __forceinline__ void dst_body(const Member* __restrict__ mems, const 
                             a4[l] = rbo[ol];
                         }
                     }
-                    double z[PQ_MAXL];
 #pragma unroll
-                    for (int l = 0; l < PQ_MAXL; ++l) {
-                        if (l < L) {
-                            double zz = 0.0;
-                            if (ok) {
-                                const long long ol = o + l * ls;
-                                // cabaret_predictor, qg3p_aux.F90:1012-1018
-                                zz = a0[l] + 0.5 * dt * a1[l];
-                                // cabaret_beta, qg3p_aux.F90:1051-1059
-                                const double rbn = dt * (0.5 * (a3[l] + a2[l]) * Mb.beta[l]);
-                                zz = zz + (1.0 + ta) * rbn - ta * a4[l];
-                                rb[ol] = (S)rbn;
-                                zp[ol] = (S)zz;
-                                if (MX) zz = (double)(S)zz;  // the stored (FP32) value
-                            }
-                            z[l] = zz;
+                    for (int l = 0; l < LC; ++l) {
+                        double zz = 0.0;
+                        if (has(l) && ok) {
+                            const long long ol = o + l * ls;
+                            zz = a0[l] + 0.5 * dt * a1[l];
+                            const double rbn = dt * (0.5 * (a3[l] + a2[l]) * Mb.beta[l]);
+                            zz = zz + (1.0 + ta) * rbn - ta * a4[l];
+                            rb[ol] = (S)rbn;
+                            zp[ol] = (S)zz;
+                            if (MX) zz = (double)(S)zz;  // the stored (FP32) value
                         }
+                        z[l] = zz;
                     }
-#pragma unroll 1
-                    for (int m = 0; m < L; ++m) {
-                        double sacc = 0.0;
+                };
+                auto project = [&](int r, int t, const double (&za)[LC], const double (&zb)[LC]) {
+                    // z_to_modes, qg3p_diagnostics.F90:545-549
+#pragma unroll ZR ? LC : 1
+                    for (int m = 0; m < LC; ++m) {
+                        if (!has(m)) break;
+                        double sa = 0.0, sb = 0.0;
 #pragma unroll
-                        for (int l = 0; l < PQ_MAXL; ++l)
-                            if (l < L) sacc += Mb.z2m[m * PQ_MAXL + l] * z[l];
-                        put(m, r, k, cff * sacc);
+                        for (int l = 0; l < LC; ++l) {
+                            if (has(l)) {
+                                const double w = ZR ? zm[ZR ? m : 0][ZR ? l : 0] : Mb.z2m[m * PQ_MAXL + l];
+                                sa += w * za[l];
+                                sb += w * zb[l];
+                            }
+                        }
+                        put(m, r, t, cff * sa, cff * sb);
+                    }
+                };
+                for (int r = 0; r < R; ++r) {
+                    const bool ok = j0 + r < jend;
+                    const int j = ok ? j0 + r : jend - 1;
+                    [[maybe_unused]] const S* row = zin + (long long)j * pitch;
+                    for (int t0 = threadIdx.x; t0 < M; t0 += nthr * UN) {
+                        double za[UN][LC], zb[UN][LC];
+                        if constexpr (PRO == PRO_STEP) {
+                            const int k = t0 ? t0 : M;
+                            step_node(j, k, ok, za[0]);
+                            if (LC > 2) asm volatile("" ::: "memory");  // one node's loads at a time
+                            if (t0) {
+                                step_node(j, N - k, ok, zb[0]);
+                            } else {
+#pragma unroll
+                                for (int l = 0; l < LC; ++l) zb[0][l] = za[0][l];
+                            }
+                        } else {
+                            S va[UN][LC], vb[UN][LC];
+#pragma unroll
+                            for (int q = 0; q < UN; ++q) {
+                                const int t = t0 + q * nthr, k = t ? t : M;
+#pragma unroll
+                                for (int l = 0; l < LC; ++l) {
+                                    const bool in = has(l) && t < M;
+                                    va[q][l] = in ? __ldg(row + l * ls + k) : (S)0;
+                                    vb[q][l] = in ? __ldg(row + l * ls + N - k) : (S)0;
+                                }
+                            }
+#pragma unroll
+                            for (int q = 0; q < UN; ++q)
+#pragma unroll
+                                for (int l = 0; l < LC; ++l) {
+                                    za[q][l] = (double)va[q][l];
+                                    zb[q][l] = (double)vb[q][l];
+                                }
+                        }
+#pragma unroll
+                        for (int q = 0; q < UN; ++q)
+                            if (t0 + q * nthr < M) project(r, t0 + q * nthr, za[q], zb[q]);
                     }
                 }
+            };
+            switch (L) {
+                case 1: rows(std::integral_constant<int, 1>{}, std::true_type{}); break;
+                case 2: rows(std::integral_constant<int, 2>{}, std::true_type{}); break;
+                case 3: rows(std::integral_constant<int, 3>{}, std::true_type{}); break;
+                case 4: rows(std::integral_constant<int, 4>{}, std::true_type{}); break;
+                case 5: rows(std::integral_constant<int, 5>{}, std::true_type{}); break;
+                default: rows(std::integral_constant<int, PQ_MAXL>{}, std::false_type{});
             }
         }
     } else {
-        // unit (m, r) entries 1..n <- spec(m, j, 0..n-1); one warp per unit row
-        for (int rm = warp; rm < R * L; rm += nwarp) {
-            const int m = rm / R, r = rm - m * R;
-            const int j = j0 + r;
-            const bool ok = (Mb.periodic || (j >= 1 && j <= jj - 2)) && j < jend;
-            if (fp64_mode(m)) {
-                const double* g = (MX ? Mb.spec64 : reinterpret_cast<const double*>(Mb.spec)) + m * ls +
-                                  (long long)(ok ? j : 1) * pitch - 1;
-                double* d = ubuf(m, r);
-                for (int k = 1 + lane; k <= n; k += 32) cp8z(d + k, g + k, ok);
-            } else if (gemm_bc) {
-                // Rows the tensor-core DST already took back to node values:
-                // straight to the positions the back-projection reads.
-                const float* g = reinterpret_cast<const float*>(Mb.gbuf) + m * ls + (long long)(ok ? j : 1) * pitch - 1;
-                float* d = reinterpret_cast<float*>(ubuf(m, r));
-                for (int k = 1 + lane; k <= n; k += 32) cp4z(d + xpad(k), g + k, ok);
-            } else {
-                const float* g = reinterpret_cast<const float*>(Mb.spec) + m * ls + (long long)(ok ? j : 1) * pitch - 1;
-                float* d = reinterpret_cast<float*>(ubuf(m, r));
-                for (int k = 1 + lane; k <= n; k += 32) cp4z(d + k, g + k, ok);
+        if (EPI == EPI_PV && corr_smem) {
+            const double* corr = Mb.corr;
+            const int cw = pitch >> 1;
+            for (int rm = warp; rm < R * (L - 1); rm += nwarp) {
+                const int r = rm / (L - 1), m = 1 + rm - r * (L - 1);
+                const int j = j0 + r;
+                const bool ok = j < jend;
+                const double* g = corr + m * ls + (long long)(ok ? j : 0) * pitch;
+                double* d = extra + (size_t)rm * pitch;
+                for (int q = lane; q < cw; q += 32) cp16(d + 2 * q, g + 2 * q, ok);
             }
+        }
+        // psic_here: this thread's first partial means, in flight with the rows.
+        const int KT = 8 / tri_warps(jj), tpm = (n + KT - 1) / KT;
+        double acc[PQ_MAXL];
+        if (EPI == EPI_PV && psic_here) {
+#pragma unroll
+            for (int mm = 0; mm < PQ_MAXL; ++mm)
+                acc[mm] = (mm < L && (int)threadIdx.x < tpm) ? __ldcg(Mb.partials + (long long)mm * tpm + threadIdx.x) : 0.0;
+        }
+        // x_k = spec(m, j, k-1); the boundary rows of a closed basin are zero.
+        const long long ro = um * ls + (long long)(interior ? ju : 1) * pitch - 1;
+        if (fp64_mode(um)) {
+            const double* g = (MX ? Mb.spec64 : reinterpret_cast<const double*>(Mb.spec)) + ro;
+            stage_unit<V>(ubuf(um, ur), p, P, N, Mb.was, [&](int k) { return interior ? __ldg(g + k) : 0.0; });
+        } else if (gemm_bc) {
+            // Rows the tensor-core DST already took back to node values:
+            // straight to the positions the back-projection reads.
+            const float* g = reinterpret_cast<const float*>(Mb.gbuf) + ro;
+            float* d = ubuf32(um, ur);
+            for (int k = 1 + p; k <= n; k += P) d[xpad(k)] = interior ? __ldg(g + k) : 0.f;
+        } else {
+            const float* g = reinterpret_cast<const float*>(Mb.spec) + ro;
+            stage_unit<V>(ubuf32(um, ur), p, P, N, Mb.was_f, [&](int k) { return interior ? __ldg(g + k) : 0.f; });
         }
         if (EPI == EPI_PV && psic_here) {
             // psiC_m = (sum of the tridiagonal CTAs' partial means of mode m)
             // / (g_ii_int g_jj_int) (modes_to_z_correct_mass,
             // qg3p_aux.F90:482-521), summed in the same fixed order by every
-            // CTA while its rows load (one pass for all modes); the member's
+            // CTA (one pass for all modes); the member's
             // first CTA publishes it and flags a NaN (the reference aborts,
             // :504-510) or a value above 1e100 (it warns, :511-517).
-            const int KT = 8 / tri_warps(jj), tpm = (n + KT - 1) / KT;
-            double acc[PQ_MAXL];
-#pragma unroll
-            for (int mm = 0; mm < PQ_MAXL; ++mm) acc[mm] = 0.0;
-            for (int q = threadIdx.x; q < tpm; q += nthr)
+            for (int q = threadIdx.x + nthr; q < tpm; q += nthr)
 #pragma unroll
                 for (int mm = 0; mm < PQ_MAXL; ++mm)
                     if (mm < L) acc[mm] += __ldcg(Mb.partials + (long long)mm * tpm + q);
@@ -634,36 +653,22 @@ __device__ __forceinline__ void dst_body(const Member* __restrict__ mems, const 
                 }
             }
         }
-        if (EPI == EPI_PV && corr_smem) {
-            const double* corr = Mb.corr;
-            const int cw = pitch >> 1;
-            for (int rm = warp; rm < R * (L - 1); rm += nwarp) {
-                const int r = rm / (L - 1), m = 1 + rm - r * (L - 1);
-                const int j = j0 + r;
-                const bool ok = j < jend;
-                const double* g = corr + m * ls + (long long)(ok ? j : 0) * pitch;
-                double* d = extra + (size_t)rm * pitch;
-                for (int q = lane; q < cw; q += 32) cp16(d + 2 * q, g + 2 * q, ok);
-            }
-        }
-        cp_commit_wait_all();
     }
-    __syncthreads();
+    // Rows staged by the whole CTA (the projection), or by the unit itself.
+    if (EPI == EPI_SPEC && PRO != PRO_PLAIN)
+        __syncthreads();
+    else
+        unit_sync(P, u);
 
     // ---------------- per-unit transform ----------------------------------
-    const int u = threadIdx.x / P, p = threadIdx.x & (P - 1);
-    const int um = u / R, ur = u - um * R;
-    const int ju = j0 + ur;
-    double* buf = ubuf(um, ur);
-    const bool interior = (Mb.periodic || (ju >= 1 && ju <= jj - 2)) && ju < jend;
     __shared__ double utot[8][2];  // cross-warp scan totals of units wider than a warp
     // With gemm_bc the baroclinic rows (a whole warp's or unit's mode) are
     // transformed by the tensor-core DST instead (pq_dst_mma.cu).
     if (fp64_mode(um))
-        dst_unit<V, double>(buf, p, P, u, utot[u & 7], N, M, logM, Mb.tw, Mb.wsplit, Mb.was);
+        dst_unit<V, PC, double>(ubuf(um, ur), p, P, u, utot[u & 7], N, M, Mb.tw, Mb.wsplit);
     else if (!gemm_bc)
-        dst_unit<V, float>(reinterpret_cast<float*>(buf), p, P, u, reinterpret_cast<float*>(utot[u & 7]), N, M, logM,
-                           Mb.tw_f, Mb.wsplit_f, Mb.was_f);
+        dst_unit<V, PC, float>(ubuf32(um, ur), p, P, u, reinterpret_cast<float*>(utot[u & 7]), N, M, Mb.tw_f, Mb.wsplit_f);
+    if (EPI == EPI_PV && corr_smem) cp_commit_wait_all();
     pdl_release();
 
     if (EPI == EPI_SPEC) {
@@ -671,15 +676,11 @@ __device__ __forceinline__ void dst_body(const Member* __restrict__ mems, const 
             if (fp64_mode(um)) {
                 double* spec = (MX ? Mb.spec64 : reinterpret_cast<double*>(Mb.spec)) + um * ls +
                                (long long)ju * pitch - 1;
+                const double* buf = ubuf(um, ur);
                 for (int k = 1 + p; k <= n; k += P) spec[k] = buf[xpad(k)];
-            } else if (gemm_bc) {
-                // node values of the projected row, for the tensor-core DST
-                float* g = reinterpret_cast<float*>(Mb.gbuf) + um * ls + (long long)ju * pitch - 1;
-                const float* fb = reinterpret_cast<const float*>(buf);
-                for (int k = 1 + p; k <= n; k += P) g[k] = fb[k];
-            } else {
+            } else if (!gemm_bc) {
                 float* spec = reinterpret_cast<float*>(Mb.spec) + um * ls + (long long)ju * pitch - 1;
-                const float* fb = reinterpret_cast<const float*>(buf);
+                const float* fb = ubuf32(um, ur);
                 for (int k = 1 + p; k <= n; k += P) spec[k] = fb[xpad(k)];
             }
         }
@@ -690,10 +691,13 @@ __device__ __forceinline__ void dst_body(const Member* __restrict__ mems, const 
         // FP32 units are widened).
         double* io = reinterpret_cast<double*>(Mb.helm_io) + um * ls + (long long)ju * pitch;
         if (interior) {
-            if (fp64_mode(um))
+            if (fp64_mode(um)) {
+                const double* buf = ubuf(um, ur);
                 for (int k = 1 + p; k <= n; k += P) io[k] = buf[xpad(k)];
-            else
-                for (int k = 1 + p; k <= n; k += P) io[k] = (double)reinterpret_cast<const float*>(buf)[xpad(k)];
+            } else {
+                const float* fb = ubuf32(um, ur);
+                for (int k = 1 + p; k <= n; k += P) io[k] = (double)fb[xpad(k)];
+            }
             if (p == 0) io[ii - 1] = 0.0;
         } else if (ju == 0 && !Mb.periodic) {
             for (int k = 1 + p; k <= n; k += P) io[k] = 0.0;
@@ -805,23 +809,26 @@ __device__ __forceinline__ void dst_body(const Member* __restrict__ mems, const 
     }
 }
 
-template <typename S, int V, int PRO, int EPI>
-__global__ void __launch_bounds__(dst_max_threads(V)) k_dst(const Member* __restrict__ mems, const int* __restrict__ prefix,
-                                                             int nmem, int row_offset, int c, int corr_smem,
-                                                             int psic_here, const __grid_constant__ Member one,
-                                                             int use_one, int gemm_bc) {
-    dst_body<S, V, PRO, EPI>(mems, prefix, nmem, row_offset, c, corr_smem, psic_here, one, use_one, gemm_bc);
+// MINB > 0: registers capped so that MINB CTAs of the bound's threads fit an
+// SM (dst_min_ctas); the bodies' widest layer counts would otherwise set the
+// register count of all.
+template <typename S, int V, int PC, int PRO, int EPI>
+__global__ void __launch_bounds__(dst_max_threads(V))
+    k_dst(const Member* __restrict__ mems, const int* __restrict__ prefix, int nmem, int row_offset, int c,
+          int corr_smem, int psic_here, const __grid_constant__ Member one, int use_one, int gemm_bc) {
+    dst_body<S, V, PC, PRO, EPI>(mems, prefix, nmem, row_offset, c, corr_smem, psic_here, one, use_one, gemm_bc);
 }
-// The inverse with 64-lane units of 8 values: registers capped so that three
-// 256-thread CTAs fit (80), hence four of its 192-thread CTAs, where its
-// back-projection would otherwise take 166 registers and allow two; the
-// epilogue spills a little.  (An explicit bound on the other instances would
-// raise their register counts, so they keep the plain one.)
-template <typename S, int V, int PRO, int EPI>
-__global__ void __launch_bounds__(dst_max_threads(V), 3)
+template <typename S, int V, int PC, int PRO, int EPI, int MINB>
+__global__ void __launch_bounds__(dst_max_threads(V), MINB)
     k_dst_capped(const Member* __restrict__ mems, const int* __restrict__ prefix, int nmem, int row_offset, int c,
                  int corr_smem, int psic_here, const __grid_constant__ Member one, int use_one, int gemm_bc) {
-    dst_body<S, V, PRO, EPI>(mems, prefix, nmem, row_offset, c, corr_smem, psic_here, one, use_one, gemm_bc);
+    dst_body<S, V, PC, PRO, EPI>(mems, prefix, nmem, row_offset, c, corr_smem, psic_here, one, use_one, gemm_bc);
+}
+// CTAs per SM the registers must allow (0: no bound): the forward DST three
+// of 256 threads up to 8 values per lane; 16 values two of 320.
+template <int V, int PRO, int EPI>
+__host__ __device__ constexpr int dst_min_ctas() {
+    return PRO == PRO_STEP ? (V <= 8 ? 2 : 0) : V == 16 ? 2 : (V <= 8 && EPI == EPI_SPEC && PRO == PRO_MODAL) ? 3 : 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -1312,22 +1319,27 @@ static int psic_in_inverse(const LaunchSet& ls) {
     return (!ls.periodic && ls.ctas_dst[1] <= 4 * ls.sm_count) ? 1 : 0;
 }
 
-template <typename S, int V, int PRO, int EPI>
+template <typename S, int V, int PC, int PRO, int EPI>
 static cudaError_t launch_dst_v(const LaunchSet& ls, cudaStream_t st) {
     const int M = ls.maxN / 2, L = ls.maxL;
     const int R = dst_rows_per_cta(M / V, ls.dst_group);
     const int threads = L * R * (M / V);
-    size_t bytes = (size_t)L * R * dst_unit_len(ls.maxN) * sizeof(double);
+    size_t bytes = dst_units_len(L, R, ls.maxN, sizeof(S) == 4) * sizeof(double);
     const size_t cbytes = (size_t)R * (L - 1) * ls.maxPitch * sizeof(double);
-    const int corr_smem = (EPI == EPI_PV && !ls.periodic && bytes + cbytes <= 200 * 1024) ? 1 : 0;
+    // corr rows in shared memory only while four CTAs still fit an SM
+    const int corr_smem = (EPI == EPI_PV && !ls.periodic && bytes + cbytes <= 56 * 1024) ? 1 : 0;
     if (corr_smem) bytes += cbytes;
-    if (sizeof(S) == 4 && EPI == EPI_SPEC && PRO != PRO_STEP)
-        bytes += (size_t)R * L * ls.maxN * (PRO == PRO_PLAIN ? sizeof(double) : sizeof(float));
     // The inverse with 64-lane units of 8 values takes the register-capped
     // instance (1025^2 x 3: 41.1 -> 37.3 us mixed, 44.5 -> 41.7 us FP64).
-    void (*kern)(const Member*, const int*, int, int, int, int, int, Member, int, int) = k_dst<S, V, PRO, EPI>;
-    if constexpr (EPI == EPI_PV && V == 8) {
-        if (M / V == 64) kern = k_dst_capped<S, V, PRO, EPI>;
+    void (*kern)(const Member*, const int*, int, int, int, int, int, Member, int, int);
+    constexpr int MINB = dst_min_ctas<V, PRO, EPI>();
+    if constexpr (MINB > 0) {
+        kern = k_dst_capped<S, V, PC, PRO, EPI, MINB>;
+    } else {
+        kern = k_dst<S, V, PC, PRO, EPI>;
+        if constexpr (EPI == EPI_PV && V == 8) {
+            if (M / V == 64) kern = k_dst_capped<S, V, PC, PRO, EPI, 3>;
+        }
     }
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return e;
@@ -1338,14 +1350,35 @@ static cudaError_t launch_dst_v(const LaunchSet& ls, cudaStream_t st) {
                               member_arg_used(ls), sizeof(S) == 4 ? ls.gemm_bc : 0);
 }
 
+// The compile-time geometries: what the defaults select (dst_lanes_default
+// for a step, dst_lanes_batched for the stand-alone solves).
 template <typename S, int PRO, int EPI>
 static cudaError_t launch_dst(const LaunchSet& ls, cudaStream_t st) {
-    switch (ls.maxN / 2 / ls.dst_lanes[EPI == EPI_SPEC ? 0 : 1]) {
-        case 2: return launch_dst_v<S, 2, PRO, EPI>(ls, st);
-        case 4: return launch_dst_v<S, 4, PRO, EPI>(ls, st);
-        case 8: return launch_dst_v<S, 8, PRO, EPI>(ls, st);
-        case 16: return launch_dst_v<S, 16, PRO, EPI>(ls, st);
-        case 32: return launch_dst_v<S, 32, PRO, EPI>(ls, st);
+    const int P = ls.dst_lanes[EPI == EPI_SPEC ? 0 : 1], V = ls.maxN / 2 / P;
+    constexpr bool STEP = PRO != PRO_PLAIN || EPI == EPI_PV;
+    constexpr bool HELM = EPI == EPI_HELM || (PRO == PRO_PLAIN && EPI == EPI_SPEC);
+    if constexpr (STEP) {
+        if (V == 2 && P == 16) return launch_dst_v<S, 2, 16, PRO, EPI>(ls, st);
+        if (V == 2 && P == 32) return launch_dst_v<S, 2, 32, PRO, EPI>(ls, st);
+        if (V == 4 && P == 32) return launch_dst_v<S, 4, 32, PRO, EPI>(ls, st);
+        if (V == 8 && P == 64) return launch_dst_v<S, 8, 64, PRO, EPI>(ls, st);
+        if (V == 16 && P == 64) return launch_dst_v<S, 16, 64, PRO, EPI>(ls, st);
+    }
+    if constexpr (HELM) {
+        if (V == 8 && P == 4) return launch_dst_v<S, 8, 4, PRO, EPI>(ls, st);
+        if (V == 8 && P == 8) return launch_dst_v<S, 8, 8, PRO, EPI>(ls, st);
+        if (V == 8 && P == 16) return launch_dst_v<S, 8, 16, PRO, EPI>(ls, st);
+        if (V == 16 && P == 32) return launch_dst_v<S, 16, 32, PRO, EPI>(ls, st);
+    }
+    if constexpr (STEP || HELM) {
+        if (V == 8 && P == 32) return launch_dst_v<S, 8, 32, PRO, EPI>(ls, st);
+    }
+    switch (V) {
+        case 2: return launch_dst_v<S, 2, 0, PRO, EPI>(ls, st);
+        case 4: return launch_dst_v<S, 4, 0, PRO, EPI>(ls, st);
+        case 8: return launch_dst_v<S, 8, 0, PRO, EPI>(ls, st);
+        case 16: return launch_dst_v<S, 16, 0, PRO, EPI>(ls, st);
+        case 32: return launch_dst_v<S, 32, 0, PRO, EPI>(ls, st);
         default: return cudaErrorInvalidValue;
     }
 }
