@@ -385,11 +385,12 @@ PQ_API int pq_energy_noalloc(const double* psi, int ii, int jj, int layers, int 
  *              layer; 1 warp sweeps down bands of cab_band rows of a
  *              32-column strip, claimed from a queue by resident warps;
  *              2 the same with two columns per lane (64-column strips; the
- *              mixed form only).  Default: tiles up to jj = 700, then
- *              sweeps; two-column sweeps in the mixed form above jj = 1500
- *   cab_band   output rows per sweep, 4..128 (default: 8 up to 300 rows,
- *              32 up to 700, then 24 (FP64) or 16 (mixed) up to 1500, and
- *              40 (FP64) or 24 (mixed) above)
+ *              mixed form only).  Default: tiles up to ii jj layers = 370000
+ *              (280000 in the mixed form), then sweeps; two-column sweeps in
+ *              the mixed form above jj = 1500
+ *   cab_band   output rows per sweep, 4..128 (default: the height whose
+ *              schedule on the device's resident warps ends first, at most
+ *              40; 24 for two-column sweeps)
  *   dst_group  row groups per DST CTA: a CTA holds dst_group * layers
  *              warps (0: automatic, 1); layers * dst_group <= 8
  *   dst_lanes, dst_lanes_inv  lanes per (row, mode) unit of the forward

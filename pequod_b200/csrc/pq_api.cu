@@ -382,20 +382,20 @@ int pq::create_ctx(pq_ctx** out, const pq_model_desc* d, int device, bool helm_o
     const size_t lstride = (size_t)c->pitch * jj;
     c->field_bytes = lstride * L * sizeof(double);
     const int ntiles_tri = tri_ctas(n, jj, L);
-    // CABARET formulation and band height by grid size (measured on B200,
-    // pq_tuning overrides): tiles up to 700 rows; above, persistent warp
-    // sweeps, two columns per lane in the mixed form beyond 1500 rows.  Bands
-    // (swept 8..48): short ones keep the end of the sweep queue short, tall
-    // ones cut halo rows -- 1025 x 1025 x 3: 24 (FP64), 16 (mixed);
-    // 2049 x 2049 x 5: 40 (FP64), 24 (mixed, two columns).
+    // CABARET formulation by grid size (measured on B200, pq_tuning
+    // overrides).  Tiles while the grid is too small to fill the resident
+    // sweep warps: 330k nodes 27.4 us against 29.2 (FP64), 198k 19.8 against
+    // 20.7 (mixed); sweeps from 395k 32.9 -> 30.7, 789k 52.5 -> 41.7 (FP64), 308k
+    // 24.7 -> 23.3, 789k 39.6 -> 32.0 (mixed).  Mixed beyond 1500 rows: two
+    // columns per lane (2049^2 x 5: 372 us against 398), in bands of 24 rows (its
+    // edge sweeps round the forcing once, so its bands are kept).
     const bool mixed = d->precision == PQ_PREC_MIXED;
-    const int cab_kernel = jj <= 700 ? 0 : (mixed && jj > 1500) ? 2 : 1;
-    const int cab_sh = jj <= 300 ? 8 : jj <= 700 ? 32 : jj <= 1500 ? (mixed ? 16 : 24) : (mixed ? 24 : 40);
+    const long long nodes = (long long)ii * jj * L;
+    const int cab_kernel = helm_only ? 0 : (mixed && jj > 1500) ? 2 : nodes < (mixed ? 280000 : 370000) ? 0 : 1;
+    const int cab_sh = helm_only ? kMinBand : cab_kernel == 2 ? 24 : cabaret_band(ii, jj, L, 1, mixed);
     const int ntiles_cab = d->periodic_j ? channel_ctas(ii, jj)
                            : cab_kernel == 0 ? cabaret_tile_ctas(ii, jj, L)
                                              : cabaret_ctas(ii, jj, L, cab_sh, cab_kernel, mixed);
-    const int ntiles_cab_max =
-        std::max({cabaret_ctas_bound(ii, jj, L, kMinBand), cabaret_tile_ctas(ii, jj, L), channel_ctas(ii, jj)});
 
     // Tables: exp(-2 pi i t / M) and exp(-2 pi i t / N), laid out the way the
     // row DST reads them (pq_helm.cu: three pass plans, five lane widths).
@@ -530,7 +530,7 @@ int pq::create_ctx(pq_ctx** out, const pq_model_desc* d, int device, bool helm_o
     const size_t o_ica = take((size_t)4 * PQ_MAXL * sizeof(double));
     const size_t npart = std::max((size_t)2 * ntiles_tri, (size_t)jj * (PQ_MAXL + 1));
     const size_t o_part = take(npart * sizeof(double));
-    const size_t o_maxu = take(ntiles_cab_max * sizeof(double));
+    const size_t o_maxu = take(sizeof(unsigned long long));
     const size_t o_cnt = take(4 * sizeof(unsigned));
     const size_t o_sc = take(sizeof(Scalars));
     const size_t o_st = take(sizeof(int));
@@ -648,7 +648,7 @@ int pq::create_ctx(pq_ctx** out, const pq_model_desc* d, int device, bool helm_o
     }
     m.wind = c->wind.empty() ? nullptr : reinterpret_cast<const double*>(A + o_wind);
     m.partials = reinterpret_cast<double*>(A + o_part);
-    m.maxu_part = reinterpret_cast<double*>(A + o_maxu);
+    m.maxu = reinterpret_cast<unsigned long long*>(A + o_maxu);
     m.counters = reinterpret_cast<unsigned*>(A + o_cnt);
     m.sc = reinterpret_cast<Scalars*>(A + o_sc);
     m.status = reinterpret_cast<int*>(A + o_st);

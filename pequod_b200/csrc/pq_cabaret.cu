@@ -24,37 +24,31 @@ namespace pq {
 // 2 halo columns on each side -- and marches down a band of Mb.cab_sh output
 // rows (a tuning parameter).  Every per-lane quantity lives in registers as
 // a rolling window over rows; the i-neighbours come from the lane's own
-// columns or, across a lane boundary, from warp shuffles.  At iteration r
-// (s = r - 2) the warp loads psi row s+2 and the inputs of rows s, s-1, and
-// produces
+// columns or, across a lane boundary, from warp shuffles.  At iteration k
+// (s = j0 + k - 2) the warp takes psi row s and the inputs of rows s, s-1, s-2,
+// and produces
 //   rel(s), zeta after BC/forcing at row s-1, uj on face row s, ui on row s-1,
-//   zeta_fj on face row s-1, zeta_fi on row s-1, and res / zeta_old at row s-2,
-// so output row o is final at iteration o + 4.
+//   zeta_fj on face row s-1, zeta_fi on row s-1, and res / zeta_old at row s-2.
 // NC = 2 (FP32 fields only, pq_tuning.cab_kernel = 2): each row access of a
 // field is one 8-byte vector per lane (16 bytes for psi) and one shuffle
-// serves two columns, 26 % fewer instructions per node than NC = 1; it needs
-// more registers (two CTAs per SM instead of three), so it pays on large
-// grids (2049^2 x 5) and not at 1025^2.
+// serves two columns; it needs more registers (two CTAs per SM instead of
+// three), so it pays on large grids (2049^2 x 5).
+//
+// What bounds it: instruction issue and latency at 12 warps per SM (issue
+// active 45-50 %, DRAM 45-65 % of its peak), and the end of the sweep queue.
+// 1025^2 x 3, us per launch, FP64 / mixed: 133 / 98 with a copy and an address
+// per lane and field, one cp.async each; 121 / 93 with the descriptor read from the kernel's
+// parameters (field bases in uniform registers), one-sided shuffles and FP64
+// max / min as selects; 120 / 90 with edge sweeps on the same iteration and
+// 16-byte copies; 107 / 75 with every wall sweep claimed first, bands sized to
+// the resident warps and the step finished by the last warp.  Bulk copies
+// (cp.async.bulk, a row of a field each) were slower (134 / 122): one lane's
+// operands at a time.  More CTAs per SM (4, 5) gave nothing at FP64 (125, 170)
+// and 2 % mixed.  513^2 x 3: 58 / 43 (tiles) -> 42 / 32; 2049^2 x 5 631 / 405 ->
+// 599 / 373.
 constexpr int CAB_WARPS = 4;
 constexpr int CAB_D = 4;  // depth of the per-warp cp.async row pipeline
-// Streamed inputs of one iteration (rows relative to s = r - 2).
-enum { F_PSI2 = 0, F_ZPB, F_PSIM, F_PSIP, F_ZO, F_UIMO, F_UJMO, F_FIO, F_FJ, F_WIND, F_RB, CAB_NF };
 __host__ __device__ constexpr int cab_sw(int nc) { return 32 * nc - 4; }  // output columns per warp
-// Ring stage layout: each field a slot of the warp's 32 NC values at their
-// own width (FP64 for psi and the wind, T for the rest), in enum order.
-__host__ __device__ constexpr bool cab_f64_field(int f) {
-    return f == F_PSI2 || f == F_PSIM || f == F_PSIP || f == F_WIND;
-}
-template <typename T, int NC>
-__host__ __device__ constexpr int cab_slot(int f) {  // offset of field f in a stage, in doubles
-    int o = 0;
-    for (int k = 0; k < f; ++k) o += cab_f64_field(k) ? 32 * NC : 32 * NC * (int)sizeof(T) / 8;
-    return o;
-}
-template <typename T, int NC>
-__host__ __device__ constexpr int cab_ring() {  // doubles per warp
-    return CAB_D * cab_slot<T, NC>(CAB_NF);
-}
 
 __device__ __forceinline__ double shup(double v, int d) { return __shfl_up_sync(0xffffffffu, v, d); }
 __device__ __forceinline__ double shdn(double v, int d) { return __shfl_down_sync(0xffffffffu, v, d); }
@@ -126,18 +120,55 @@ __device__ __forceinline__ void vst(V* p, const V (&v)[NC]) {
         *reinterpret_cast<float2*>(p) = make_float2(v[0], v[1]);
     }
 }
-template <int BYTES>
-__device__ __forceinline__ void cp_async_ca(unsigned dst, const void* src, int src_bytes) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(dst), "l"(src), "n"(BYTES), "r"(src_bytes)
+// z + f r, the forcing added to zeta.  FP32 written out, so that a mixed run
+// does not depend on what the compiler contracts: the product rounded first,
+// as in the tile kernel.  `once` rounds the sum only: the second column of a
+// two-column edge sweep has always done so, and is kept bit for bit.
+__device__ __forceinline__ double add_scaled(double z, double f, double r, bool) { return z + f * r; }
+__device__ __forceinline__ float add_scaled(float z, float f, float r, bool once) {
+    return once ? __fmaf_rn(f, r, z) : __fadd_rn(z, __fmul_rn(f, r));
+}
+// max / min as one comparison and a select: FP64 fmax is a sequence around the
+// NaN rules, which the limiter does not need (a NaN in any of its inputs is in
+// zeta too and poisons the next inversion).
+__device__ __forceinline__ double mx(double a, double b) { return a > b ? a : b; }
+__device__ __forceinline__ double mn(double a, double b) { return a < b ? a : b; }
+__device__ __forceinline__ float mx(float a, float b) { return fmaxf(a, b); }
+__device__ __forceinline__ float mn(float a, float b) { return fminf(a, b); }
+// The input rows of an iteration come in 16-byte chunks (cp.async.cg: no line of the L1 cache
+// is held while a copy is in flight; the 8-byte copies of the edge sweep hold
+// three lines each, and the L1 cache left beside the rings bounds how many
+// fly).  The rows of an iteration lie one after another in a ring stage --
+// first the FP64 ones, then the T ones -- and instruction q of a class copies
+// chunks 32 q .. 32 q + 31 of them: a lane's chunk belongs to one field for
+// the whole sweep, so its address is one pointer that moves a row down per
+// iteration.  T = float rows start two columns early and are four values
+// longer, so that every chunk starts on 16 bytes (i0 is a multiple of 28 or 60).
+enum { G_PSI = 0, G_PSIM, G_PSIP, G_WIND, G_N64 };
+enum { G_ZPB = 0, G_ZO, G_UIMO, G_UJMO, G_FIO, G_FJ, G_RB, G_NT };
+template <typename T, int NC> struct CabRing {
+    static constexpr int LEAD = sizeof(T) == 4 ? 2 : 0;
+    static constexpr int B64 = 32 * NC * 8, BT = (32 * NC + 2 * LEAD) * (int)sizeof(T);  // bytes of a row
+    static constexpr int C64 = G_N64 * B64 / 16, CT = G_NT * BT / 16;                    // chunks of a stage
+    static constexpr int Q64 = (C64 + 31) / 32, QT = (CT + 31) / 32;                     // copy instructions
+    static constexpr int STAGE = G_N64 * B64 + G_NT * BT;
+    __host__ __device__ static constexpr int bytes() { return CAB_D * STAGE; }
+};
+__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+template <int OFF>
+__device__ __forceinline__ void cp_chunk(unsigned dst, const void* src, unsigned bytes) {  // bytes 0: zeros
+    asm volatile("cp.async.cg.shared.global [%0+%2], [%1], 16, %3;\n" ::"r"(dst), "l"(src), "n"(OFF), "r"(bytes)
                  : "memory");
 }
 
 // One warp's sweep over layer l of the strip starting at column i0 and the
-// band starting at row j0.  EDGE = false is the specialisation for warps
-// whose whole footprint (columns i0-2 .. i0+32NC-3, rows j0-4 .. j0+sh+3)
-// lies at least two nodes inside the domain: no bounds checks, no boundary
-// branches, vector loads and stores.  PRED = true also applies the next
-// step's cabaret_predictor and cabaret_beta (fixed dt) to every interior
+// band of rows j0 .. j0+SH-1.  EDGE = false is the specialisation for warps
+// whose whole footprint (columns i0-2 .. i0+32NC-3, rows j0-4 .. j0+SH+3) lies
+// at least two nodes inside the domain; EDGE = true runs the same iteration
+// and replaces what differs at the walls (rows by warp-uniform branches, the
+// columns of a strip that touches a wall per lane), masking values outside
+// the domain to zero.  PRED = true also applies the next step's
+// cabaret_predictor and cabaret_beta (fixed dt) to every interior
 // node it finishes, writing the next step's inversion input zeta_next and
 // res_beta_other.  T is the type of the CABARET fields (double, or float in
 // the mixed form); psi is FP64 and everything computed from psi differences
@@ -145,76 +176,121 @@ __device__ __forceinline__ void cp_async_ca(unsigned dst, const void* src, int s
 // velocities before the time weighting) is evaluated in FP64.  Returns the
 // largest |u| of the faces it wrote.
 template <bool EDGE, bool PRED, typename T, int NC>
-__device__ __forceinline__ double cab_sweep(const Member& Mb, int l, int i0, int j0, int lane, double* ring) {
+__device__ __forceinline__ double cab_sweep(const Member& Mb, int l, int i0, int j0, int SH, int lane, char* ring) {
     static_assert(NC == 1 || NC == 2, "one or two columns per lane");
-    const int ii = Mb.ii, jj = Mb.jj, L = Mb.L, pitch = Mb.pitch;
+    using RG = CabRing<T, NC>;
+    const int L = Mb.L, pitch = Mb.pitch, ii = Mb.ii, jj = Mb.jj;
     const long long ls = Mb.lstride;
-    const int ib = i0 - 2 + NC * lane;  // the lane's first column
-    int ic[NC];
-    bool in_i[NC];
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-        ic[c] = ib + c;
-        in_i[c] = !EDGE || (ic[c] >= 0 && ic[c] < ii);
-    }
     constexpr int HL = 2 / NC;  // halo lanes on each side
-    // Owner lanes of their columns' nodes, i-faces (a = i) and j-faces.
     const bool out_lane = lane >= HL && lane < 32 - HL;
     const int cur = Mb.cur, nxt = cur ^ 1;
     const double dt64 = Mb.sc->dt;
     const T dt = (T)dt64, tu = (T)Mb.sc->tweight_u;
     const bool avg = cab_average_gate(Mb);
-    double* const psi_av = Mb.psi_av;
     const T hdt = (T)0.5 * dt;
-    const int SH = Mb.cab_sh;
-    // All fields of a member live in one allocation: address them by 32-bit
-    // element offsets from one base (fewer live registers than 16 pointers);
-    // FP64 fields (psi, wind) from B, T fields from BT.  Every field starts
-    // on a 256-byte boundary and rows are a multiple of 32 values apart, so
-    // the lane's NC values (from an even column when NC = 2) are aligned for
-    // one vector access.
-    const double* B = Mb.psi;
-    const T* BT = reinterpret_cast<const T*>(B);
-    auto ofs = [&](const void* f) { return (int)(reinterpret_cast<const double*>(f) - B); };
-    auto ofst = [&](const void* f) { return (int)(reinterpret_cast<const T*>(f) - BT); };
-    const int lo = (int)(l * ls) + ib;  // layer and column part of every offset
-    const int o_psil = lo;
-    const int o_psim = (l > 0) ? lo - (int)ls : lo;
-    const int o_psip = (l < L - 1) ? lo + (int)ls : lo;
-    const int o_zpb = ofst(Mb.zeta) + lo;
-    const int o_zo = ofst(Mb.zeta_old[cur]) + lo;
-    const int o_zn = ofst(Mb.zeta_old[nxt]) + lo;
-    const int o_res = ofst(Mb.res_out) + lo;
-    const int o_ui = ofst(Mb.ui) + lo;
-    const int o_uj = ofst(Mb.uj) + lo;
-    const int o_uimo = ofst(Mb.uimo[cur]) + lo;
-    const int o_uimon = ofst(Mb.uimo[nxt]) + lo;
-    const int o_ujmo = ofst(Mb.ujmo[cur]) + lo;
-    const int o_ujmon = ofst(Mb.ujmo[nxt]) + lo;
-    const int o_fio = ofst(Mb.zfi[cur]) + lo;
-    const int o_fin = ofst(Mb.zfi[nxt]) + lo;
-    const int o_fjo = ofst(Mb.zfj[cur]) + lo;
-    const int o_fjn = ofst(Mb.zfj[nxt]) + lo;
-    const int o_rb = PRED ? ofst(Mb.res_beta) + lo : 0;
-    const int o_rbn = PRED ? ofst(Mb.res_beta_other) + lo : 0;
-    const int o_zpn = PRED ? ofst(Mb.zeta_next) + lo : 0;
     const T ta = (T)Mb.sc->tweight_a, beta_l = (T)Mb.beta[l];
     const bool has_wind = (l == 0 && Mb.wind);
-    const int o_wind = has_wind ? ofs(Mb.wind) + ib : 0;
-    T* W = const_cast<T*>(BT);
     const T nu = (T)Mb.viscosity, vb = (T)Mb.visc_bot;
     const double s1 = Mb.s1[l], s2 = Mb.s2[l];
-    const int bc = Mb.bc_type;
-    const double cffbc = Mb.alpha / (Mb.alpha + 3.0);
     const bool lim = Mb.limiter != 0;
     const bool top = (l == 0), bottom = (l == L - 1);
     T umax = 0;  // |u| is exact in T: widened once at the end
+    const int ib = i0 - 2 + NC * lane;  // the lane's first column
+    // Column masks (true inside): nodes, interior nodes, i-faces a = i.
+    auto in_i = [&](int c) { return !EDGE || (ib + c >= 0 && ib + c < ii); };
+    auto int_i = [&](int c) { return !EDGE || (ib + c >= 1 && ib + c <= ii - 2); };
+    auto fac_i = [&](int c) { return !EDGE || (ib + c >= 1 && ib + c <= ii - 1); };
+    auto in_j = [&](int j) { return !EDGE || (j >= 0 && j < jj); };
+    auto int_j = [&](int j) { return !EDGE || (j >= 1 && j <= jj - 2); };
+    const bool walls = EDGE && (i0 - 2 <= 0 || i0 + 32 * NC - 3 >= ii - 1);  // the strip holds a wall column
+    const int bc = Mb.bc_type;
+    const double cffbc = Mb.alpha / (Mb.alpha + 3.0);
 
-    auto ld = [&](int off, int row, int c) -> double {
-        if (EDGE) return (in_i[c] && row >= 0 && row < jj) ? B[off + c + row * pitch] : 0.0;
-        return B[off + c + row * pitch];
+    // This lane's chunks: their addresses at the next row to copy, and 16 or,
+    // where the field does not exist, 0 bytes.
+    const int n = SH + 4;
+    const char *c64[RG::Q64], *cT[RG::QT];
+    unsigned b64[RG::Q64], bT[RG::QT];
+    int r64[RG::Q64], rT[RG::QT];  // EDGE: the row the chunk comes from at the next copy
+#pragma unroll
+    for (int q = 0; q < RG::Q64; ++q) {
+        const int c = 32 * q + lane, f = c * 16 / RG::B64, col = (c * 16 % RG::B64) / 8;
+        const bool on = f == G_PSI || (f == G_PSIM && !top) || (f == G_PSIP && !bottom) || (f == G_WIND && has_wind);
+        const int layer = f == G_WIND ? 0 : f == G_PSIM ? l - 1 : f == G_PSIP ? l + 1 : l;
+        const double* base = f == G_WIND ? Mb.wind : Mb.psi;
+        r64[q] = j0 - 2 - (f == G_WIND ? 1 : 0);
+        // Outside the row (a chunk lies wholly inside or outside it): zeros.
+        const bool ok = on && (!EDGE || (i0 - 2 + col >= 0 && i0 - 2 + col < pitch));
+        b64[q] = ok ? 16u : 0u;
+        c64[q] = reinterpret_cast<const char*>(ok ? base + layer * ls + (long long)r64[q] * pitch + (i0 - 2 + col)
+                                                  : Mb.psi);
+    }
+#pragma unroll
+    for (int q = 0; q < RG::QT; ++q) {
+        const int c = 32 * q + lane, f = c * 16 / RG::BT, col = (c * 16 % RG::BT) / (int)sizeof(T);
+        const void* base = f == G_ZPB    ? Mb.zeta
+                           : f == G_ZO   ? Mb.zeta_old[cur]
+                           : f == G_UIMO ? Mb.uimo[cur]
+                           : f == G_UJMO ? Mb.ujmo[cur]
+                           : f == G_FIO  ? Mb.zfi[cur]
+                           : f == G_FJ   ? Mb.zfj[cur]
+                                         : Mb.res_beta;
+        const int d = f == G_RB ? 2 : (f == G_ZO || f == G_UIMO || f == G_FIO) ? 1 : 0;  // rows above s
+        const bool on = f < G_RB || (f == G_RB && PRED);
+        rT[q] = j0 - 2 - d;
+        const int gc = i0 - 2 - RG::LEAD + col;
+        const bool ok = on && (!EDGE || (gc >= 0 && gc < pitch));
+        bT[q] = ok ? 16u : 0u;
+        cT[q] = reinterpret_cast<const char*>(ok ? static_cast<const T*>(base) + l * ls + (long long)rT[q] * pitch + gc
+                                                 : static_cast<const T*>(Mb.zeta));
+    }
+    const unsigned p64 = (unsigned)pitch * 8u, pT = (unsigned)pitch * (unsigned)sizeof(T);
+    const unsigned ring_a = smem_addr(ring) + 16u * lane;
+    auto issue = [&](int k) {
+        const unsigned dst = ring_a + (unsigned)(k % CAB_D) * RG::STAGE;
+        // chunk 32 q + lane of each class, the last instruction's lanes past its end left out
+#define PQ_CP64(q)                                                                     \
+    if constexpr (q < RG::Q64) {                                                       \
+        const bool in = !EDGE || (r64[q] >= 0 && r64[q] < jj);                         \
+        if (32 * q + 32 <= RG::C64 || 32 * q + lane < RG::C64)                         \
+            cp_chunk<512 * q>(dst, in ? c64[q] : reinterpret_cast<const char*>(Mb.psi), in ? b64[q] : 0u); \
+        c64[q] += b64[q] ? p64 : 0u;                                                   \
+        ++r64[q];                                                                      \
+    }
+#define PQ_CPT(q)                                                                      \
+    if constexpr (q < RG::QT) {                                                        \
+        const bool in = !EDGE || (rT[q] >= 0 && rT[q] < jj);                           \
+        if (32 * q + 32 <= RG::CT || 32 * q + lane < RG::CT)                           \
+            cp_chunk<G_N64 * RG::B64 + 512 * q>(dst, in ? cT[q] : reinterpret_cast<const char*>(Mb.psi), \
+                                                in ? bT[q] : 0u);                      \
+        cT[q] += bT[q] ? pT : 0u;                                                      \
+        ++rT[q];                                                                       \
+    }
+        PQ_CP64(0) PQ_CP64(1) PQ_CP64(2) PQ_CP64(3)
+        PQ_CPT(0) PQ_CPT(1) PQ_CPT(2) PQ_CPT(3)
+#undef PQ_CP64
+#undef PQ_CPT
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
-    // rel_from_zeta_and_psi coupling for an interior node.
+    static_assert(RG::Q64 <= 4 && RG::QT <= 4, "copy instructions per stage");
+    for (int k = 0; k < CAB_D - 1; ++k) issue(k);  // n > CAB_D - 1 (SH >= 1)
+
+    // Output addresses: element (row, this lane's first column) of a field.
+    const long long lo = l * ls + ib;
+    T* const p_res = reinterpret_cast<T*>(Mb.res_out) + lo;
+    T* const p_zn = reinterpret_cast<T*>(Mb.zeta_old[nxt]) + lo;
+    T* const p_rbn = reinterpret_cast<T*>(Mb.res_beta_other) + lo;
+    T* const p_zpn = reinterpret_cast<T*>(Mb.zeta_next) + lo;
+    T* const p_ui = reinterpret_cast<T*>(Mb.ui) + lo;
+    T* const p_uimon = reinterpret_cast<T*>(Mb.uimo[nxt]) + lo;
+    T* const p_fin = reinterpret_cast<T*>(Mb.zfi[nxt]) + lo;
+    T* const p_uj = reinterpret_cast<T*>(Mb.uj) + lo;
+    T* const p_ujmon = reinterpret_cast<T*>(Mb.ujmo[nxt]) + lo;
+    T* const p_fjn = reinterpret_cast<T*>(Mb.zfj[nxt]) + lo;
+    double* const p_av = Mb.psi_av + lo;
+    const double* const p_psi = Mb.psi + lo;
+
+    // rel_from_zeta_and_psi coupling.
     auto rel_int = [&](T z, double p, double pm, double pp) -> T {
         if (L == 1) return z;
         if (top) return (T)((double)z + s2 * (p - pp));
@@ -230,87 +306,35 @@ __device__ __forceinline__ double cab_sweep(const Member& Mb, int l, int i0, int
         const T d_f = -(psi_n - psi_o) * (T)2 - dt * v0 * dfi;
         T v = (T)2 * psi_n - fi2;
         if (lim) {
-            const T fmx = fmax(fmax(fi1, fi2), psi_n) - d_f;
-            const T fmn = fmin(fmin(fi1, fi2), psi_n) - d_f;
-            if (v > fmx) v = fmx;
-            if (v < fmn) v = fmn;
-        }
-        return v;
-    };
-    // The wall branch of the extrapolator: upwind node on the boundary.
-    auto extrap_wall = [&](T fi1, T psi_n, T psi_o) -> T {
-        const T fi2 = psi_n;
-        const T d_f = -(psi_n - psi_o);
-        T v = (T)2 * psi_n - fi2;
-        if (lim) {
-            const T fmx = fmax(fmax(fi1, fi2), psi_n) - d_f;
-            const T fmn = fmin(fmin(fi1, fi2), psi_n) - d_f;
+            const T fmx = mx(mx(fi1, fi2), psi_n) - d_f;
+            const T fmn = mn(mn(fi1, fi2), psi_n) - d_f;
             if (v > fmx) v = fmx;
             if (v < fmn) v = fmn;
         }
         return v;
     };
 
-    // Row copies of iteration r into ring stage r % CAB_D: per field one
-    // cp.async of the lane's NC values (interior warps), or one per value
-    // (edge warps: values outside the domain, and zeta at non-interior nodes,
-    // are zero-filled by a source size of 0, the source then the field base).
-    // Slots: cab_slot (each field at its own width).
-    constexpr int STAGE = cab_slot<T, NC>(CAB_NF);
-    constexpr int S_PSI2 = cab_slot<T, NC>(F_PSI2), S_ZPB = cab_slot<T, NC>(F_ZPB), S_PSIM = cab_slot<T, NC>(F_PSIM),
-                  S_PSIP = cab_slot<T, NC>(F_PSIP), S_ZO = cab_slot<T, NC>(F_ZO), S_UIMO = cab_slot<T, NC>(F_UIMO),
-                  S_UJMO = cab_slot<T, NC>(F_UJMO), S_FIO = cab_slot<T, NC>(F_FIO), S_FJ = cab_slot<T, NC>(F_FJ),
-                  S_WIND = cab_slot<T, NC>(F_WIND), S_RB = cab_slot<T, NC>(F_RB);
-    auto cp64 = [&](double* slot, int off, int row) {
-        const unsigned sa = (unsigned)__cvta_generic_to_shared(slot + NC * lane);
-        if (!EDGE) {
-            cp_async_ca<8 * NC>(sa, B + (off + row * pitch), 8 * NC);
-        } else {
-            const bool rok = row >= 0 && row < jj;
-#pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                const bool ok = rok && in_i[c];
-                cp_async_ca<8>(sa + 8u * c, ok ? B + (off + c + row * pitch) : B, ok ? 8 : 0);
-            }
+    // The wall branch: upwind node on the boundary.
+    auto extrap_wall = [&](T fi1, T psi_n, T psi_o) -> T {
+        const T fi2 = psi_n;
+        const T d_f = -(psi_n - psi_o);
+        T v = (T)2 * psi_n - fi2;
+        if (lim) {
+            const T fmx = mx(mx(fi1, fi2), psi_n) - d_f;
+            const T fmn = mn(mn(fi1, fi2), psi_n) - d_f;
+            if (v > fmx) v = fmx;
+            if (v < fmn) v = fmn;
         }
+        return v;
     };
-    auto cpt = [&](double* slot, int off, int row, bool node_int) {
-        const unsigned sa = (unsigned)__cvta_generic_to_shared(reinterpret_cast<T*>(slot) + NC * lane);
-        if (!EDGE) {
-            cp_async_ca<(int)sizeof(T) * NC>(sa, BT + (off + row * pitch), (int)sizeof(T) * NC);
-        } else {
-            const bool rok = node_int ? (row > 0 && row < jj - 1) : (row >= 0 && row < jj);
-#pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                const bool ok = rok && (node_int ? (ic[c] > 0 && ic[c] < ii - 1) : in_i[c]);
-                cp_async_ca<(int)sizeof(T)>(sa + (unsigned)sizeof(T) * c, ok ? BT + (off + c + row * pitch) : BT,
-                                            ok ? (int)sizeof(T) : 0);
-            }
-        }
+    // apply_rel_bc from the wall node and the two nodes inward.
+    auto rel_wall = [&](double p, double q1, double q2) -> T {
+        if (bc == 3) return (T)0;
+        return (T)((bc == 1) ? cffbc * (-3.5 * p + 4.0 * q1 - 0.5 * q2) : 2.0 * (q1 - p));
     };
-    auto issue = [&](int rr) {
-        const int ss = rr - 2;
-        double* d = ring + (rr % CAB_D) * STAGE;
-        cp64(d + S_PSI2, o_psil, ss + 2);
-        cpt(d + S_ZPB, o_zpb, ss, true);
-        if (L > 1) {
-            cp64(d + S_PSIM, o_psim, ss);
-            cp64(d + S_PSIP, o_psip, ss);
-        }
-        cpt(d + S_ZO, o_zo, ss - 1, false);
-        cpt(d + S_UIMO, o_uimo, ss - 1, false);
-        cpt(d + S_UJMO, o_ujmo, ss, false);
-        cpt(d + S_FIO, o_fio, ss - 1, false);
-        cpt(d + S_FJ, o_fjo, ss, false);
-        if (has_wind) cp64(d + S_WIND, o_wind, ss - 1);
-        if (PRED) cpt(d + S_RB, o_rb, ss - 2, false);
-    };
-    for (int rr = j0; rr < j0 + CAB_D - 1; ++rr) {
-        issue(rr);
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-    }
+
     // Rolling windows.
-    double P0[NC], P1[NC], P2[NC], P3[NC], P4[NC];
+    double P1[NC], P2[NC];  // psi rows s-1, s
     T Rm2[NC], Rm1[NC];    // rel rows s-2, s-1
     T ZFm2[NC];            // zeta after forcing, row s-2
     T ZOm2[NC];            // zeta_old row s-2
@@ -320,61 +344,52 @@ __device__ __forceinline__ double cab_sweep(const Member& Mb, int l, int i0, int
     T FLI[NC];             // flux_i row s-2 (face a = i)
     T UIm2[NC];            // ui row s-2 (face a = i)
     T zpb_prev[NC];
-    double pm_prev[NC], pp_prev[NC], pe_prev[NC];
+    double pe_prev[NC];
+    [[maybe_unused]] double pm_prev[NC], pp_prev[NC];  // EDGE: psi of the neighbour layers, row s-1
 #pragma unroll
     for (int c = 0; c < NC; ++c) {
-        P0[c] = 0;
-        P1[c] = ld(o_psil, j0 - 4, c);
-        P2[c] = ld(o_psil, j0 - 3, c);
-        P3[c] = ld(o_psil, j0 - 2, c);
-        P4[c] = ld(o_psil, j0 - 1, c);
+        P2[c] = (in_j(j0 - 3) && in_i(c)) ? p_psi[(long long)(j0 - 3) * pitch + c] : 0.0;
         Rm2[c] = Rm1[c] = ZFm2[c] = ZOm2[c] = UJm2[c] = UJm1[c] = FJm2[c] = FJm1[c] = FLJm2[c] = FLI[c] = UIm2[c] =
             zpb_prev[c] = 0;
-        pm_prev[c] = pp_prev[c] = pe_prev[c] = 0;
+        pe_prev[c] = pm_prev[c] = pp_prev[c] = 0;
     }
     // The left neighbour of P1 (psi row s-1) is, for the lane's first column,
     // the previous row's left neighbour of P2 (carried over, so the corner
     // needs no second shuffle), for the others the lane's own column.
     double up1_prev0 = shup(P2[NC - 1], 1);
 
-    const int rend = j0 + SH + 4;
 #pragma unroll 1
-    for (int r = j0; r < rend; ++r) {
-        const int s = r - 2;
-        // ---- loads -----------------------------------------------------------
-        // Keep CAB_D - 1 iterations of row copies in flight.
-        if (r + CAB_D - 1 < rend) issue(r + CAB_D - 1);
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-        asm volatile("cp.async.wait_group %0;\n" ::"n"(CAB_D - 1) : "memory");
-        const double* st = ring + (r % CAB_D) * STAGE;
-        auto get64 = [&](int so, double(&v)[NC]) { vld<NC>(st + so + NC * lane, v); };
-        auto gett = [&](int so, T(&v)[NC]) { vld<NC>(reinterpret_cast<const T*>(st + so) + NC * lane, v); };
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-            P0[c] = P1[c];
-            P1[c] = P2[c];
-            P2[c] = P3[c];
-            P3[c] = P4[c];
-        }
-        get64(S_PSI2, P4);
+    for (int k = 0; k < n; ++k) {
+        const int s = j0 + k - 2;
+        // Row k's copies have landed: this lane's (wait), then everyone's (the
+        // barrier, which also ends the reads of the stage refilled next).
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(CAB_D - 2) : "memory");
+        __syncwarp();
+        if (k + CAB_D - 1 < n)
+            issue(k + CAB_D - 1);
+        else
+            asm volatile("cp.async.commit_group;\n" ::: "memory");
+        const char* st = ring + (k % CAB_D) * RG::STAGE;
+        auto get64 = [&](int f, double(&v)[NC]) { vld<NC>(reinterpret_cast<const double*>(st + f * RG::B64) + NC * lane, v); };
+        auto gett = [&](int f, T(&v)[NC]) {
+            vld<NC>(reinterpret_cast<const T*>(st + G_N64 * RG::B64 + f * RG::BT) + RG::LEAD + NC * lane, v);
+        };
         T zpb_s[NC], zo_1[NC], uimo_1[NC], ujmo_s[NC], fio_1[NC], fj_s[NC], w_1[NC], rb_2[NC];
         double pm_s[NC], pp_s[NC];
-        gett(S_ZPB, zpb_s);
-        if (L > 1) {
-            get64(S_PSIM, pm_s);
-            get64(S_PSIP, pp_s);
-        } else {
 #pragma unroll
-            for (int c = 0; c < NC; ++c) pm_s[c] = pp_s[c] = 0.0;
-        }
-        gett(S_ZO, zo_1);
-        gett(S_UIMO, uimo_1);
-        gett(S_UJMO, ujmo_s);
-        gett(S_FIO, fio_1);
-        gett(S_FJ, fj_s);
+        for (int c = 0; c < NC; ++c) P1[c] = P2[c];
+        get64(G_PSI, P2);
+        get64(G_PSIM, pm_s);  // not read by a layer without that neighbour
+        get64(G_PSIP, pp_s);
+        gett(G_ZPB, zpb_s);
+        gett(G_ZO, zo_1);
+        gett(G_UIMO, uimo_1);
+        gett(G_UJMO, ujmo_s);
+        gett(G_FIO, fio_1);
+        gett(G_FJ, fj_s);
         if (has_wind) {
             double w[NC];
-            get64(S_WIND, w);
+            get64(G_WIND, w);
 #pragma unroll
             for (int c = 0; c < NC; ++c) w_1[c] = (T)w[c];
         } else {
@@ -382,45 +397,43 @@ __device__ __forceinline__ double cab_sweep(const Member& Mb, int l, int i0, int
             for (int c = 0; c < NC; ++c) w_1[c] = (T)0;
         }
         if (PRED) {
-            gett(S_RB, rb_2);
+            gett(G_RB, rb_2);
         } else {
 #pragma unroll
             for (int c = 0; c < NC; ++c) rb_2[c] = (T)0;
         }
 
         // ---- rel(s): rel_from_zeta_and_psi + apply_rel_bc -------------------
-        double up1[NC], up2[NC], dn1[NC], dn2[NC];
+        double up1[NC];
         col_up(P2, up1);
-        if (EDGE) {
-            col_up2(P2, up2);
-            col_dn(P2, dn1);
-            col_dn2(P2, dn2);
-        }
         T rel_s[NC];
 #pragma unroll
-        for (int c = 0; c < NC; ++c) {
-            rel_s[c] = 0;
-            if (!EDGE) {
-                rel_s[c] = rel_int(zpb_s[c], P2[c], pm_s[c], pp_s[c]);
-            } else if (in_i[c] && s >= 0 && s < jj) {
-                const int i = ic[c];
-                const bool bj = (s == 0 || s == jj - 1), bi = (i == 0 || i == ii - 1);
-                if (bj || bi) {
-                    if (bc != 3) {
-                        double q1, q2;
-                        if (bj) {
-                            q1 = (s == 0) ? P3[c] : P1[c];
-                            q2 = (s == 0) ? P4[c] : P0[c];
-                        } else {
-                            q1 = (i == 0) ? dn1[c] : up1[c];
-                            q2 = (i == 0) ? dn2[c] : up2[c];
-                        }
-                        rel_s[c] = (T)((bc == 1) ? cffbc * (-3.5 * P2[c] + 4.0 * q1 - 0.5 * q2) : 2.0 * (q1 - P2[c]));
+        for (int c = 0; c < NC; ++c) rel_s[c] = rel_int(zpb_s[c], P2[c], pm_s[c], pp_s[c]);
+        if constexpr (EDGE) {
+            // Walls (apply_rel_bc; the corners take the j-wall's formula,
+            // which the reference applies last).
+            if (s == 0 || s == jj - 1) {
+                const long long d = s == 0 ? pitch : -(long long)pitch;
+#pragma unroll
+                for (int c = 0; c < NC; ++c)
+                    if (in_i(c)) {
+                        const double* p = p_psi + (long long)s * pitch + c;
+                        rel_s[c] = rel_wall(P2[c], p[d], p[2 * d]);
                     }
-                } else {
-                    rel_s[c] = rel_int(zpb_s[c], P2[c], pm_s[c], pp_s[c]);
+            } else if (walls) {
+                double up2[NC], dn1[NC], dn2[NC];
+                col_up2(P2, up2);
+                col_dn(P2, dn1);
+                col_dn2(P2, dn2);
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    if (ib + c == 0) rel_s[c] = rel_wall(P2[c], dn1[c], dn2[c]);
+                    if (ib + c == ii - 1) rel_s[c] = rel_wall(P2[c], up1[c], up2[c]);
                 }
             }
+#pragma unroll
+            for (int c = 0; c < NC; ++c)
+                if (!(in_j(s) && in_i(c))) rel_s[c] = 0;
         }
 
         // ---- zeta at row s-1 after update_zeta_bc and cabaret_forcing -------
@@ -431,32 +444,30 @@ __device__ __forceinline__ double cab_sweep(const Member& Mb, int l, int i0, int
         T zf_1[NC];
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
-            zf_1[c] = 0;
-            const int i = ic[c];
-            if (!EDGE || (in_i[c] && s1r >= 0 && s1r < jj)) {
-                const bool bnd = EDGE && (s1r == 0 || s1r == jj - 1 || i == 0 || i == ii - 1);
-                if (bnd) {
-                    if (L == 1)
-                        zf_1[c] = Rm1[c];
-                    else if (top)
-                        zf_1[c] = (T)((double)Rm1[c] - s2 * (P1[c] - pp_prev[c]));
-                    else if (bottom)
-                        zf_1[c] = (T)((double)Rm1[c] - s1 * (P1[c] - pm_prev[c]));
-                    else
-                        zf_1[c] = (T)((double)Rm1[c] - s1 * (P1[c] - pm_prev[c]) - s2 * (P1[c] - pp_prev[c]));
-                } else {
-                    const T lap = (T)-4 * Rm1[c] + rl_up[c] + rl_dn[c] + Rm2[c] + rel_s[c];
-                    T rv;
-                    if (L == 1)
-                        rv = dt * (w_1[c] - vb * Rm1[c] + nu * lap);
-                    else if (top)
-                        rv = dt * (w_1[c] + nu * lap);
-                    else if (bottom)
-                        rv = dt * (-vb * Rm1[c] + nu * lap);
-                    else
-                        rv = dt * nu * lap;
-                    zf_1[c] = zpb_prev[c] + rv;
-                }
+            const T lap = (T)-4 * Rm1[c] + rl_up[c] + rl_dn[c] + Rm2[c] + rel_s[c];
+            T fr, f = dt;  // the forcing is f * fr
+            if (L == 1) {
+                fr = w_1[c] - vb * Rm1[c] + nu * lap;
+            } else if (top) {
+                fr = w_1[c] + nu * lap;
+            } else if (bottom) {
+                fr = -vb * Rm1[c] + nu * lap;
+            } else {
+                f = dt * nu;
+                fr = lap;
+            }
+            zf_1[c] = add_scaled(zpb_prev[c], f, fr, EDGE && c == 1);
+            if (EDGE && !(int_j(s1r) && int_i(c))) {
+                if (!(in_j(s1r) && in_i(c)))
+                    zf_1[c] = 0;
+                else if (L == 1)
+                    zf_1[c] = Rm1[c];
+                else if (top)
+                    zf_1[c] = (T)((double)Rm1[c] - s2 * (P1[c] - pp_prev[c]));
+                else if (bottom)
+                    zf_1[c] = (T)((double)Rm1[c] - s1 * (P1[c] - pm_prev[c]));
+                else
+                    zf_1[c] = (T)((double)Rm1[c] - s1 * (P1[c] - pm_prev[c]) - s2 * (P1[c] - pp_prev[c]));
             }
         }
 
@@ -470,73 +481,67 @@ __device__ __forceinline__ double cab_sweep(const Member& Mb, int l, int i0, int
         for (int c = 0; c < NC; ++c) pe_here[c] = 0.25 * (P2[c] + P1[c] + up1[c] + left1[c]);
         col_dn(pe_here, pe_dn);
         T uj_s[NC], ujm_s[NC], ui_1[NC], uim_1[NC];
-        bool fj_ok[NC], fi_ok[NC];
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
-            const int i = ic[c];
-            uj_s[c] = ujm_s[c] = 0;  // face b = s, column i
-            fj_ok[c] = !EDGE || (s >= 1 && s <= jj - 1 && i >= 1 && i <= ii - 2);
-            if (fj_ok[c]) {
-                ujm_s[c] = (T)(pe_dn[c] - pe_here[c]);
-                uj_s[c] = ((T)1 + tu) * ujm_s[c] - tu * ujmo_s[c];
-            }
-            ui_1[c] = uim_1[c] = 0;  // row s-1, face a = i
-            fi_ok[c] = !EDGE || (i >= 1 && i <= ii - 1 && s1r >= 1 && s1r <= jj - 2);
-            if (fi_ok[c]) {
-                uim_1[c] = (T)(-pe_here[c] + pe_prev[c]);
-                ui_1[c] = ((T)1 + tu) * uim_1[c] - tu * uimo_1[c];
-            }
+            ujm_s[c] = (T)(pe_dn[c] - pe_here[c]);  // face b = s
+            uj_s[c] = ((T)1 + tu) * ujm_s[c] - tu * ujmo_s[c];
+            uim_1[c] = (T)(-pe_here[c] + pe_prev[c]);  // row s-1, face a = i
+            ui_1[c] = ((T)1 + tu) * uim_1[c] - tu * uimo_1[c];
+            if (EDGE && !(s >= 1 && s <= jj - 1 && int_i(c))) uj_s[c] = ujm_s[c] = 0;
+            if (EDGE && !(int_j(s1r) && fac_i(c))) ui_1[c] = uim_1[c] = 0;
         }
 
         // ---- extrapolator, j-faces: face b = s-1 -------------------------------
         T fjn[NC];
-        bool bfj_ok[NC];
-        const int bf = s - 1;
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
-            fjn[c] = 0;
-            bfj_ok[c] = !EDGE || (bf >= 1 && bf <= jj - 1 && ic[c] >= 1 && ic[c] <= ii - 2);
-            if (bfj_ok[c]) {
-                const T u1 = UJm1[c];
-                const bool pos = u1 >= (T)0;
-                if (!EDGE)
-                    fjn[c] = extrap(u1, pos ? UJm2[c] : uj_s[c], FJm1[c], pos ? FJm2[c] : fj_s[c],
-                                    pos ? ZFm2[c] : zf_1[c], pos ? ZOm2[c] : zo_1[c], pos);
-                else if (pos)
-                    fjn[c] = bf > 1 ? extrap(u1, UJm2[c], FJm1[c], FJm2[c], ZFm2[c], ZOm2[c], true)
-                                    : extrap_wall(FJm1[c], ZFm2[c], ZOm2[c]);
-                else
-                    fjn[c] = bf < jj - 1 ? extrap(u1, uj_s[c], FJm1[c], fj_s[c], zf_1[c], zo_1[c], false)
-                                         : extrap_wall(FJm1[c], zf_1[c], zo_1[c]);
+            const T u1 = UJm1[c];
+            const bool pos = u1 >= (T)0;
+            fjn[c] = extrap(u1, pos ? UJm2[c] : uj_s[c], FJm1[c], pos ? FJm2[c] : fj_s[c], pos ? ZFm2[c] : zf_1[c],
+                            pos ? ZOm2[c] : zo_1[c], pos);
+            if (EDGE) {
+                if (s1r == 1 && pos) fjn[c] = extrap_wall(FJm1[c], ZFm2[c], ZOm2[c]);
+                if (s1r == jj - 1 && !pos) fjn[c] = extrap_wall(FJm1[c], zf_1[c], zo_1[c]);
+                if (!(s1r >= 1 && s1r <= jj - 1 && int_i(c))) fjn[c] = 0;
             }
         }
 
         // ---- extrapolator, i-faces on row s-1: face a = i ------------------------
-        T ui_up[NC], ui_dn[NC], fi_up[NC], fi_dn[NC], zf_up[NC], zo_up[NC];
-        col_up(ui_1, ui_up);
-        col_dn(ui_1, ui_dn);
-        col_up(fio_1, fi_up);
-        col_dn(fio_1, fi_dn);
-        col_up(zf_1, zf_up);
-        col_up(zo_1, zo_up);
         T fin[NC], flj_1[NC], fli_1[NC];
+        if constexpr (NC == 1) {
+            // The upwind side only: one shuffle from the lane that holds it.
+            const bool pos = ui_1[0] >= (T)0;
+            const int sf = pos ? lane - 1 : lane + 1, sn = pos ? lane - 1 : lane;
+            const T u2 = __shfl_sync(0xffffffffu, ui_1[0], sf), f2 = __shfl_sync(0xffffffffu, fio_1[0], sf);
+            const T zn = __shfl_sync(0xffffffffu, zf_1[0], sn), zo = __shfl_sync(0xffffffffu, zo_1[0], sn);
+            fin[0] = extrap(ui_1[0], u2, fio_1[0], f2, zn, zo, pos);
+            if (EDGE) {
+                if (walls && ((ib == 1 && pos) || (ib == ii - 1 && !pos))) fin[0] = extrap_wall(fio_1[0], zn, zo);
+                if (!(int_j(s1r) && fac_i(0))) fin[0] = 0;
+            }
+        } else {
+            T ui_up[NC], ui_dn[NC], fi_up[NC], fi_dn[NC], zf_up[NC], zo_up[NC];
+            col_up(ui_1, ui_up);
+            col_dn(ui_1, ui_dn);
+            col_up(fio_1, fi_up);
+            col_dn(fio_1, fi_dn);
+            col_up(zf_1, zf_up);
+            col_up(zo_1, zo_up);
 #pragma unroll
-        for (int c = 0; c < NC; ++c) {
-            fin[c] = 0;
-            if (fi_ok[c]) {
-                const int i = ic[c];
+            for (int c = 0; c < NC; ++c) {
                 const T u1 = ui_1[c];
                 const bool pos = u1 >= (T)0;
-                if (!EDGE)
-                    fin[c] = extrap(u1, pos ? ui_up[c] : ui_dn[c], fio_1[c], pos ? fi_up[c] : fi_dn[c],
-                                    pos ? zf_up[c] : zf_1[c], pos ? zo_up[c] : zo_1[c], pos);
-                else if (pos)
-                    fin[c] = i > 1 ? extrap(u1, ui_up[c], fio_1[c], fi_up[c], zf_up[c], zo_up[c], true)
-                                   : extrap_wall(fio_1[c], zf_up[c], zo_up[c]);
-                else
-                    fin[c] = i < ii - 1 ? extrap(u1, ui_dn[c], fio_1[c], fi_dn[c], zf_1[c], zo_1[c], false)
-                                        : extrap_wall(fio_1[c], zf_1[c], zo_1[c]);
+                fin[c] = extrap(u1, pos ? ui_up[c] : ui_dn[c], fio_1[c], pos ? fi_up[c] : fi_dn[c],
+                                pos ? zf_up[c] : zf_1[c], pos ? zo_up[c] : zo_1[c], pos);
+                if (EDGE) {
+                    if (walls && ((ib + c == 1 && pos) || (ib + c == ii - 1 && !pos)))
+                        fin[c] = extrap_wall(fio_1[c], pos ? zf_up[c] : zf_1[c], pos ? zo_up[c] : zo_1[c]);
+                    if (!(int_j(s1r) && fac_i(c))) fin[c] = 0;
+                }
             }
+        }
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
             flj_1[c] = UJm1[c] * fjn[c];  // flux_j on face s-1
             fli_1[c] = ui_1[c] * fin[c];  // flux_i on row s-1, face i
         }
@@ -545,23 +550,15 @@ __device__ __forceinline__ double cab_sweep(const Member& Mb, int l, int i0, int
         const int o = s - 2;
         T fli_dn[NC], ui_e[NC];  // flux_i and (PRED) ui on face a = i + 1, row o
         col_dn(FLI, fli_dn);
-        if (PRED) {
-            col_dn(UIm2, ui_e);
-        } else {
-#pragma unroll
-            for (int c = 0; c < NC; ++c) ui_e[c] = (T)0;
-        }
-        if ((o >= j0 && o < j0 + SH) && (!EDGE || (o >= 0 && o < jj))) {
+        if (PRED) col_dn(UIm2, ui_e);
+        const bool row_o = o >= j0 && in_j(o), row_i = s1r >= j0 && s1r < j0 + SH, row_j = s >= j0 && s < j0 + SH;
+        if (row_o) {
             T z[NC], rr[NC], zz[NC], rbn[NC];
-            bool bnd[NC];
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
-                const int i = ic[c];
-                bnd[c] = EDGE && (o == 0 || o == jj - 1 || i == 0 || i == ii - 1);
                 rr[c] = -(fli_dn[c] - FLI[c] + flj_1[c] - FLJm2[c]);
                 z[c] = ZFm2[c];
-                if (!bnd[c]) z[c] = z[c] + hdt * rr[c];
-                zz[c] = rbn[c] = 0;
+                if (int_j(o) && int_i(c)) z[c] = z[c] + hdt * rr[c];
                 if (PRED) {
                     // Next step: cabaret_predictor (qg3p_aux.F90:1012-1018) and
                     // cabaret_beta (:1051-1059) with this step's ui.
@@ -570,73 +567,69 @@ __device__ __forceinline__ double cab_sweep(const Member& Mb, int l, int i0, int
                     zz[c] = zz[c] + ((T)1 + ta) * rbn[c] - ta * rb_2[c];
                 }
             }
-            const int ro = o * pitch;
-            if (!EDGE) {
-                if (out_lane) {
-                    vst<NC>(W + (o_res + ro), rr);
-                    if (PRED) {
-                        vst<NC>(W + (o_rbn + ro), rbn);
-                        vst<NC>(W + (o_zpn + ro), zz);
-                    }
-                    vst<NC>(W + (o_zn + ro), z);
+            const long long ro = (long long)o * pitch;
+            if (out_lane && !EDGE) {
+                vst<NC>(p_res + ro, rr);
+                if (PRED) {
+                    vst<NC>(p_rbn + ro, rbn);
+                    vst<NC>(p_zpn + ro, zz);
                 }
-            } else {
+                vst<NC>(p_zn + ro, z);
+            }
+            if (out_lane && EDGE) {
 #pragma unroll
                 for (int c = 0; c < NC; ++c) {
-                    if (out_lane && in_i[c]) {
-                        if (!bnd[c]) {
-                            W[o_res + c + ro] = rr[c];
-                            if (PRED) {
-                                W[o_rbn + c + ro] = rbn[c];
-                                W[o_zpn + c + ro] = zz[c];
-                            }
+                    if (!in_i(c)) continue;
+                    if (int_j(o) && int_i(c)) {
+                        p_res[ro + c] = rr[c];
+                        if (PRED) {
+                            p_rbn[ro + c] = rbn[c];
+                            p_zpn[ro + c] = zz[c];
                         }
-                        W[o_zn + c + ro] = z[c];
                     }
+                    p_zn[ro + c] = z[c];
                 }
             }
             if (avg && out_lane) {
 #pragma unroll
                 for (int c = 0; c < NC; ++c)
-                    if (in_i[c]) psi_av[o_psil + c + ro] += dt64 * B[o_psil + c + ro];
+                    if (in_i(c)) p_av[ro + c] += dt64 * p_psi[ro + c];
             }
         }
         // ---- owned face writes ---------------------------------------------------
-        const bool row_i = s1r >= j0 && s1r < j0 + SH, row_j = s >= j0 && s < j0 + SH, row_b = bf >= j0 && bf < j0 + SH;
-        if (!EDGE) {
-            if (out_lane) {
+        if (out_lane) {
+            const long long ri = (long long)s1r * pitch;
+            if (!EDGE) {
                 if (row_i) {
-                    vst<NC>(W + (o_ui + s1r * pitch), ui_1);
-                    vst<NC>(W + (o_uimon + s1r * pitch), uim_1);
-                    vst<NC>(W + (o_fin + s1r * pitch), fin);
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) umax = fmax(umax, fabs(ui_1[c]));
+                    vst<NC>(p_ui + ri, ui_1);
+                    vst<NC>(p_uimon + ri, uim_1);
+                    vst<NC>(p_fin + ri, fin);
+                    vst<NC>(p_fjn + ri, fjn);
                 }
                 if (row_j) {
-                    vst<NC>(W + (o_uj + s * pitch), uj_s);
-                    vst<NC>(W + (o_ujmon + s * pitch), ujm_s);
-#pragma unroll
-                    for (int c = 0; c < NC; ++c) umax = fmax(umax, fabs(uj_s[c]));
+                    vst<NC>(p_uj + ri + pitch, uj_s);
+                    vst<NC>(p_ujmon + ri + pitch, ujm_s);
                 }
-                if (row_b) vst<NC>(W + (o_fjn + bf * pitch), fjn);
+            } else {
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    if (row_i && int_j(s1r) && fac_i(c)) {
+                        p_ui[ri + c] = ui_1[c];
+                        p_uimon[ri + c] = uim_1[c];
+                        p_fin[ri + c] = fin[c];
+                    }
+                    if (row_i && s1r >= 1 && s1r <= jj - 1 && int_i(c)) p_fjn[ri + c] = fjn[c];
+                    if (row_j && s >= 1 && s <= jj - 1 && int_i(c)) {
+                        p_uj[ri + pitch + c] = uj_s[c];
+                        p_ujmon[ri + pitch + c] = ujm_s[c];
+                    }
+                }
             }
-        } else {
+            // (EDGE: faces outside the domain are zero)
 #pragma unroll
             for (int c = 0; c < NC; ++c) {
-                if (out_lane && in_i[c]) {
-                    if (fi_ok[c] && row_i) {
-                        W[o_ui + c + s1r * pitch] = ui_1[c];
-                        W[o_uimon + c + s1r * pitch] = uim_1[c];
-                        W[o_fin + c + s1r * pitch] = fin[c];
-                        umax = fmax(umax, fabs(ui_1[c]));
-                    }
-                    if (fj_ok[c] && row_j) {
-                        W[o_uj + c + s * pitch] = uj_s[c];
-                        W[o_ujmon + c + s * pitch] = ujm_s[c];
-                        umax = fmax(umax, fabs(uj_s[c]));
-                    }
-                    if (bfj_ok[c] && row_b) W[o_fjn + c + bf * pitch] = fjn[c];
-                }
+                if (row_i) umax = fmax(umax, fabs(ui_1[c]));
+                if (row_j) umax = fmax(umax, fabs(uj_s[c]));
             }
         }
         // ---- shift the windows ---------------------------------------------------
@@ -654,24 +647,29 @@ __device__ __forceinline__ double cab_sweep(const Member& Mb, int l, int i0, int
             FLI[c] = fli_1[c];
             UIm2[c] = ui_1[c];
             zpb_prev[c] = zpb_s[c];
-            pm_prev[c] = pm_s[c];
-            pp_prev[c] = pp_s[c];
             pe_prev[c] = pe_here[c];
+            if (EDGE) {
+                pm_prev[c] = pm_s[c];
+                pp_prev[c] = pp_s[c];
+            }
         }
         up1_prev0 = up1[0];
     }
     return (double)umax;
 }
 
-// Last CTA of a member: max |u| over the CTAs' partial maxima, the CFL
-// number, model time, and when adaptive stepping is on dt and the time
+template <typename T, int NC>
+__host__ __device__ constexpr int cab_ring_bytes() {  // of a warp
+    return (CabRing<T, NC>::bytes() + 127) / 128 * 128;
+}
+
+// End of a member's step, by the thread that counted last: the CFL number,
+// model time, and when adaptive stepping is on dt and the time
 // weights for the next step (cabaret_cfl / cabaret_adapt_dt,
 // qg3p_aux.F90:920-990).
-// Called by every thread of the last CTA; red: shared scratch of blockDim/32.
-__device__ void finish_step(const Member& Mb, double* red) {
-    __threadfence();
-    const double mu = block_max_l2(Mb.maxu_part, Mb.ntiles_cab, red);
-    if (threadIdx.x != 0) return;
+__device__ __forceinline__ void finish_step(const Member& Mb) {
+    // max |u|, taken out for the next step
+    const double mu = __longlong_as_double((long long)atomicExch(Mb.maxu, 0ull));
     Scalars* sc = Mb.sc;
     if (cab_average_gate(Mb)) sc->diag_time += sc->dt;
     sc->max_u = mu;
@@ -696,6 +694,16 @@ __device__ void finish_step(const Member& Mb, double* red) {
     Mb.counters[1] = 0u;
     Mb.counters[3] = 0u;  // the sweep queue of k_cabaret_fused
 }
+// One thread per unit of work (a warp or a CTA, `units` of them per member)
+// reports its largest |u|: an integer maximum on the bits of the non-negative
+// value, so the result does not depend on the order.  True for the last one.
+// (Partial maxima per CTA, reduced by the last CTA, left the GPU idle for
+// 4 us at the end of every step at 1025 nodes.)
+__device__ __forceinline__ bool count_done(const Member& Mb, double umax, unsigned units) {
+    if (umax > 0.0) atomicMax(Mb.maxu, (unsigned long long)__double_as_longlong(umax));
+    __threadfence();
+    return atomicAdd(&Mb.counters[1], 1u) == units - 1u;
+}
 
 // Three CTAs per SM (at most 168 registers) with one column per lane:
 // measured 16 % faster than the unconstrained allocation (two CTAs) at
@@ -708,25 +716,39 @@ __device__ void finish_step(const Member& Mb, double* red) {
 // empty instead of idling in partly filled CTAs and waves.  The boundary
 // bands (bounds checks and boundary branches: slower) are claimed first, so
 // the last sweeps claimed are interior ones.  The last CTA resets the counter.
-template <bool PRED, typename T, int NC>
+template <bool ONE>
+__device__ __forceinline__ const Member& member_ref(const Member& smem, const Member& param) {
+    if constexpr (ONE)
+        return param;
+    else
+        return smem;
+}
+template <bool PRED, typename T, int NC, bool ONE>
 __global__ void __launch_bounds__(CAB_WARPS * 32, NC == 2 ? 2 : 3)
     k_cabaret_fused(const Member* __restrict__ mems, const int* __restrict__ prefix, int nmem,
                     const __grid_constant__ Member one, int use_one) {
-    __shared__ Member Mb;
-    __shared__ double red[CAB_WARPS];
-    __shared__ int is_last;
-    extern __shared__ __align__(16) double cab_smem[];  // [CAB_WARPS][cab_ring<T, NC>()]
+    __shared__ Member Mb_s;
+    extern __shared__ __align__(128) char cab_smem[];  // [CAB_WARPS][cab_ring_bytes<T, NC>()]
     pdl_wait();
-    int local;
-    cta_member(Mb, one, use_one, mems, prefix, nmem, blockIdx.x, &local);
-    __syncthreads();
+    int local = blockIdx.x;
+    if constexpr (!ONE) {
+        cta_member(Mb_s, one, use_one, mems, prefix, nmem, blockIdx.x, &local);
+        __syncthreads();
+    }
+    const Member& Mb = member_ref<ONE>(Mb_s, one);
     const int ii = Mb.ii, jj = Mb.jj, L = Mb.L;
     const int SH = Mb.cab_sh;
     constexpr int SW = cab_sw(NC);
     const int nstrips = (ii + SW - 1) / SW, nbands = (jj + SH - 1) / SH;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ntasks = nstrips * nbands * L;
-    double* ring = cab_smem + warp * cab_ring<T, NC>();
+    // Interior sweeps: footprint columns i0-2 .. i0+32NC-3, rows j0-4 ..
+    // j0+SH+3 at least two nodes inside the domain -- strips sA .. sA+nsi-1
+    // of bands bA .. bA+nbi-1; the nedge others (per layer) are claimed first.
+    const int sA = (4 + SW - 1) / SW, bA = (6 + SH - 1) / SH;
+    const int nsi = max(0, (ii - 32 * NC) / SW - sA + 1) * (ii >= 32 * NC), nbi = max(0, (jj - 6 - SH) / SH - bA + 1) * (jj >= 6 + SH);
+    const int nedge = nsi * nbi ? nstrips * nbands - nsi * nbi : nstrips * nbands;
+    char* ring = cab_smem + warp * cab_ring_bytes<T, NC>();
     double umax = 0.0;
     for (;;) {
         int task = 0;
@@ -734,37 +756,34 @@ __global__ void __launch_bounds__(CAB_WARPS * 32, NC == 2 ? 2 : 3)
         task = __shfl_sync(0xffffffffu, task, 0);
         if (task >= ntasks) break;
         const int l = task % L;
-        const int sb = task / L;
-        const int strip = sb % nstrips, bq = sb / nstrips;
-        const int band = nbands < 3 ? bq : bq == 0 ? 0 : bq == 1 ? nbands - 1 : bq - 1;
+        int sb = task / L, strip, band;
+        const bool interior = sb >= nedge;
+        if (interior) {
+            sb -= nedge;
+            strip = sA + sb % nsi;
+            band = bA + sb / nsi;
+        } else if (sb < (nbands - nbi) * nstrips) {  // bands at the j-walls
+            const int q = sb / nstrips;
+            strip = sb - q * nstrips;
+            band = q < bA ? q : q + nbi;
+        } else {  // strips at the i-walls
+            sb -= (nbands - nbi) * nstrips;
+            const int q = sb / nbi;
+            strip = q < sA ? q : q + nsi;
+            band = bA + sb - q * nbi;
+        }
         const int i0 = strip * SW, j0 = band * SH;
-        // Footprint: columns i0-2 .. i0+32NC-3, rows j0-4 .. j0+SH+3.
-        const bool interior =
-            (i0 - 2 >= 2) && (i0 + 32 * NC - 3 <= ii - 3) && (j0 - 4 >= 2) && (j0 + SH + 3 <= jj - 3);
-        const double u = interior ? cab_sweep<false, PRED, T, NC>(Mb, l, i0, j0, lane, ring)
-                                  : cab_sweep<true, PRED, T, NC>(Mb, l, i0, j0, lane, ring);
+        const double u = interior ? cab_sweep<false, PRED, T, NC>(Mb, l, i0, j0, SH, lane, ring)
+                                  : cab_sweep<true, PRED, T, NC>(Mb, l, i0, j0, min(SH, jj - j0), lane, ring);
         umax = fmax(umax, u);
         __syncwarp();  // the ring's last reads before the next sweep's copies
     }
     pdl_release();
 
     // Max |u| of the new face velocities (cabaret_cfl / cabaret_adapt_dt);
-    // the last CTA of the member finishes the reduction and, when adaptive
-    // time stepping is on, sets dt and the time weights for the next step
-    // (cabaret_adapt_dt, qg3p_aux.F90:946-990).
+    // the last warp of the member finishes the step.
     umax = warp_max(umax);
-    if (lane == 0) red[warp] = umax;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int w = 0; w < CAB_WARPS; ++w) t = fmax(t, red[w]);
-        Mb.maxu_part[local] = t;
-        __threadfence();
-        const unsigned prev = atomicAdd(&Mb.counters[1], 1u);
-        is_last = (prev == (unsigned)(Mb.ntiles_cab - 1));
-    }
-    __syncthreads();
-    if (is_last) finish_step(Mb, red);
+    if (lane == 0 && count_done(Mb, umax, (unsigned)(CAB_WARPS * Mb.ntiles_cab))) finish_step(Mb);
 }
 
 // ---------------------------------------------------------------------------
@@ -804,9 +823,8 @@ template <bool PRED, bool EDGE, typename T>
 // step at 513^2 x 3, +2.6 % at 257^2); every scalar the later stages need is
 // read before (the last CTA may advance them once every CTA has counted).
 // FP32 (64-80 registers, where the extra live values cost more: -5 % at 513^2)
-// counts at the end.  *is_last is set by thread 0 at the end.
-__device__ __forceinline__ void cab_tile(const Member& Mb, int l, int i0, int j0, char* smem, double* red,
-                                         int* is_last, int local) {
+// counts at the end.
+__device__ __forceinline__ void cab_tile(const Member& Mb, int l, int i0, int j0, char* smem, double* red) {
     const int ii = Mb.ii, jj = Mb.jj, L = Mb.L, pitch = Mb.pitch;
     const long long ls = Mb.lstride;
     const int cur = Mb.cur, nxt = cur ^ 1;
@@ -1112,7 +1130,7 @@ __device__ __forceinline__ void cab_tile(const Member& Mb, int l, int i0, int j0
         }
         sUj[q] = u;
     }
-    unsigned prev = 0u;
+    bool last = false;
     auto count = [&]() {
         umax = warp_max(umax);
         if (lane == 0) red[warp] = umax;
@@ -1120,9 +1138,7 @@ __device__ __forceinline__ void cab_tile(const Member& Mb, int l, int i0, int j0
         if (threadIdx.x == 0) {
             double m = 0.0;
             for (int w = 0; w < CT_THREADS / 32; ++w) m = fmax(m, red[w]);
-            Mb.maxu_part[local] = m;
-            __threadfence();
-            prev = atomicAdd(&Mb.counters[1], 1u);
+            last = count_done(Mb, m, (unsigned)Mb.ntiles_cab);
         }
     };
     if constexpr (EARLY)
@@ -1212,7 +1228,7 @@ __device__ __forceinline__ void cab_tile(const Member& Mb, int l, int i0, int j0
         zn_g[o] = z;
     }
     if constexpr (!EARLY) count();
-    if (threadIdx.x == 0) *is_last = (prev == (unsigned)(Mb.ntiles_cab - 1));
+    if (last) finish_step(Mb);
 }
 
 // MINB: CTAs per SM the register allocation must allow.  Three (80
@@ -1225,7 +1241,6 @@ __global__ void __launch_bounds__(CT_THREADS, MINB) k_cabaret_tile(const Member*
                                                               const __grid_constant__ Member one, int use_one) {
     __shared__ Member Mb;
     __shared__ double red[CT_THREADS / 32];
-    __shared__ int is_last;
     extern __shared__ __align__(16) char tsm[];
     pdl_wait();
     int local;
@@ -1240,24 +1255,22 @@ __global__ void __launch_bounds__(CT_THREADS, MINB) k_cabaret_tile(const Member*
     // the interior nodes.
     const bool inner = i0 - 2 >= 1 && i0 + CT_X + 1 <= ii - 2 && j0 - 2 >= 1 && j0 + CT_Y + 1 <= jj - 2;
     if (inner)
-        cab_tile<PRED, false, T>(Mb, l, i0, j0, tsm, red, &is_last, local);
+        cab_tile<PRED, false, T>(Mb, l, i0, j0, tsm, red);
     else
-        cab_tile<PRED, true, T>(Mb, l, i0, j0, tsm, red, &is_last, local);
+        cab_tile<PRED, true, T>(Mb, l, i0, j0, tsm, red);
     pdl_release();
-    __syncthreads();
-    if (is_last) finish_step(Mb, red);
 }
 
 // CTAs of k_cabaret_fused resident on the current device at once (at least 1).
 template <typename T, int NC>
 static int cabaret_resident_t() {
-    const size_t bytes = (size_t)CAB_WARPS * cab_ring<T, NC>() * sizeof(double);
+    const size_t bytes = (size_t)CAB_WARPS * cab_ring_bytes<T, NC>();
     int dev = 0, sms = 0, per = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaFuncSetAttribute(k_cabaret_fused<true, T, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) !=
+        cudaFuncSetAttribute(k_cabaret_fused<true, T, NC, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) !=
             cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_cabaret_fused<true, T, NC>, CAB_WARPS * 32, bytes) !=
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_cabaret_fused<true, T, NC, true>, CAB_WARPS * 32, bytes) !=
             cudaSuccess) {
         cudaGetLastError();
         return 1;
@@ -1265,18 +1278,53 @@ static int cabaret_resident_t() {
     return std::max(1, per * sms);
 }
 
-int cabaret_ctas_bound(int ii, int jj, int L, int min_sh) {
-    const int sw = cab_sw(1), nstrips = (ii + sw - 1) / sw, nbands = (jj + min_sh - 1) / min_sh;
-    return (nstrips * nbands * L + CAB_WARPS - 1) / CAB_WARPS;
+static int cabaret_resident(int nc, bool f32) {
+    return !f32 ? cabaret_resident_t<double, 1>() : nc == 2 ? cabaret_resident_t<float, 2>() : cabaret_resident_t<float, 1>();
+}
+
+// Band height: the one whose greedy schedule ends first.  A sweep of SH rows
+// costs SH + 4 iterations and about one more to start; one at a wall costs
+// up to 1.5 times an interior one (measured, 513 and 1025 nodes) and is claimed
+// earlier.  With W resident warps, floor(nE / W) or one more edge sweep each,
+// the interior sweeps then fill whole rounds: the end is the first time at
+// which every round begun so far holds them all.  At most 40 rows: taller
+// bands measured slower at 2049^2 x 5 (86 rows 661 us, 29 rows 601), where
+// the L2 cache no longer holds a row from one band to the next.
+int cabaret_band(int ii, int jj, int L, int nc, bool f32) {
+    const long long W = (long long)CAB_WARPS * cabaret_resident(nc, f32);
+    const int sw = cab_sw(nc), ns = (ii + sw - 1) / sw;
+    double best = 1e300;
+    int band = 4;
+    for (int sh = 4; sh <= 40; ++sh) {
+        const int nb = (jj + sh - 1) / sh;
+        const int nsi = ii < 32 * nc ? 0 : std::max(0, (ii - 32 * nc) / sw - (4 + sw - 1) / sw + 1);
+        const int nbi = jj < 6 + sh ? 0 : std::max(0, (jj - 6 - sh) / sh - (6 + sh - 1) / sh + 1);
+        const long long nI = (long long)nsi * nbi * L, nE = (long long)ns * nb * L - nI;
+        const double c = sh + 5, e = 1.5 * c;
+        const double a0 = e * (double)(nE / W), a1 = a0 + e;  // W - g1 warps are free at a0, g1 at a1
+        const long long g1 = nE % W, g0 = W - g1;
+        double t = g1 ? a1 : a0;
+        if (nI > 0) {
+            for (long long k0 = 0, k1 = 0; g0 * k0 + g1 * k1 < nI;) {
+                if (a0 + c * (double)(k0 + 1) <= a1 + c * (double)(k1 + 1))
+                    t = std::max(t, a0 + c * (double)++k0);
+                else
+                    t = std::max(t, a1 + c * (double)++k1);
+            }
+        }
+        if (t <= best) {
+            best = t;
+            band = sh;
+        }
+    }
+    return band;
 }
 
 int cabaret_ctas(int ii, int jj, int L, int sh, int nc, bool f32) {
     const int sw = cab_sw(nc);
     const int nstrips = (ii + sw - 1) / sw, nbands = (jj + sh - 1) / sh;
     const int need = (nstrips * nbands * L + CAB_WARPS - 1) / CAB_WARPS;
-    const int resident = !f32 ? cabaret_resident_t<double, 1>()
-                         : nc == 2 ? cabaret_resident_t<float, 2>()
-                                   : cabaret_resident_t<float, 1>();
+    const int resident = cabaret_resident(nc, f32);
     return std::min(need, resident);
 }
 
@@ -1286,15 +1334,12 @@ int cabaret_tile_ctas(int ii, int jj, int L) {
 
 template <bool PRED, typename T, int NC>
 static cudaError_t launch_sweeps(const LaunchSet& ls, cudaStream_t st) {
-    const size_t bytes = (size_t)CAB_WARPS * cab_ring<T, NC>() * sizeof(double);
-    cudaError_t e =
-        cudaFuncSetAttribute(k_cabaret_fused<PRED, T, NC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    const size_t bytes = (size_t)CAB_WARPS * cab_ring_bytes<T, NC>();
+    auto kern = member_arg_used(ls) ? k_cabaret_fused<PRED, T, NC, true> : k_cabaret_fused<PRED, T, NC, false>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return e;
-    cudaError_t le = launch_step_kernel(ls.pdl, k_cabaret_fused<PRED, T, NC>, dim3(ls.ctas_cab),
-                                        dim3(CAB_WARPS * 32), bytes, st, ls.members, ls.prefix_cab, ls.nmem,
-                                        member_arg(ls), member_arg_used(ls));
-    if (le != cudaSuccess) return le;
-    return cudaGetLastError();
+    return launch_step_kernel(ls.pdl, kern, dim3(ls.ctas_cab), dim3(CAB_WARPS * 32), bytes, st, ls.members,
+                              ls.prefix_cab, ls.nmem, member_arg(ls), member_arg_used(ls));
 }
 
 template <bool PRED, typename T>
@@ -1524,7 +1569,6 @@ template <typename T>
 __global__ void __launch_bounds__(128) k_ch_corrector(const Member* __restrict__ mems, const int* __restrict__ prefix,
                                                        int nmem) {
     __shared__ double red[4];
-    __shared__ int is_last;
     int local;
     const int mi = find_member(prefix, nmem, blockIdx.y, &local);
     const Member& Mb = mems[mi];
@@ -1564,14 +1608,8 @@ __global__ void __launch_bounds__(128) k_ch_corrector(const Member* __restrict__
     if (threadIdx.x == 0) {
         double t = 0.0;
         for (int w = 0; w < 4; ++w) t = fmax(t, red[w]);
-        const int cta = blockIdx.x + gridDim.x * local;
-        Mb.maxu_part[cta] = t;
-        __threadfence();
-        const unsigned prev = atomicAdd(&Mb.counters[1], 1u);
-        is_last = (prev == (unsigned)(Mb.ntiles_cab - 1));
+        if (count_done(Mb, t, (unsigned)Mb.ntiles_cab)) finish_step(Mb);
     }
-    __syncthreads();
-    if (is_last) finish_step(Mb, red);
 }
 
 }  // namespace

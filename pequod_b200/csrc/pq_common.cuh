@@ -130,7 +130,7 @@ struct Member {
     const double* inv_corr_a;  // [L][4], column-major 2 x 2
     const double* wind;
     double* partials;     // [L * ntiles_tri]
-    double* maxu_part;    // [ntiles_cab]
+    unsigned long long* maxu;  // max |u| of the running step, as the bits of a non-negative double; 0 between steps
     unsigned int* counters;  // [4] last-block counters
     Scalars* sc;
     int* status;
@@ -278,19 +278,6 @@ __device__ __forceinline__ double warp_max(double v) {
 // fence), and the result is valid in thread 0.  The sum has a fixed order
 // (per-thread strided sums, warp butterflies, warps in order), so it does not
 // depend on which CTA finished last.  red: shared scratch of blockDim/32.
-__device__ __forceinline__ double block_max_l2(const double* p, int n, double* red) {
-    double m = 0.0;
-    for (int q = threadIdx.x; q < n; q += blockDim.x) m = fmax(m, __ldcg(p + q));
-    m = warp_max(m);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-    __syncthreads();
-    double r = 0.0;
-    if (threadIdx.x == 0)
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) r = fmax(r, red[w]);
-    __syncthreads();
-    return r;
-}
-
 __device__ __forceinline__ double block_sum_l2(const double* p, int n, long long stride, double* red) {
     double s = 0.0;
     for (int q = threadIdx.x; q < n; q += blockDim.x) s += __ldcg(p + q * stride);

@@ -87,8 +87,8 @@ cudaError_t launch_quad(const LaunchSet& ls, int f32, int lf, cudaStream_t st);
 // CTAs of the (persistent) sweep kernel per member: band height sh, nc
 // columns per lane, FP32 fields when f32; at most the CTAs resident at once.
 int cabaret_ctas(int ii, int jj, int L, int sh, int nc, bool f32);
-// An upper bound of cabaret_ctas over every tuning with bands of at least min_sh rows.
-int cabaret_ctas_bound(int ii, int jj, int L, int min_sh);
+// The default band height of that kernel.
+int cabaret_band(int ii, int jj, int L, int nc, bool f32);
 int cabaret_tile_ctas(int ii, int jj, int L);     // CTAs of the tile kernel per member
 cudaError_t launch_rel(const LaunchSet& ls, int f32, cudaStream_t st);
 cudaError_t launch_init_finish(const LaunchSet& ls, int f32, cudaStream_t st);
