@@ -716,13 +716,6 @@ __device__ __forceinline__ bool count_done(const Member& Mb, double umax, unsign
 // empty instead of idling in partly filled CTAs and waves.  The boundary
 // bands (bounds checks and boundary branches: slower) are claimed first, so
 // the last sweeps claimed are interior ones.  The last CTA resets the counter.
-template <bool ONE>
-__device__ __forceinline__ const Member& member_ref(const Member& smem, const Member& param) {
-    if constexpr (ONE)
-        return param;
-    else
-        return smem;
-}
 template <bool PRED, typename T, int NC, bool ONE>
 __global__ void __launch_bounds__(CAB_WARPS * 32, NC == 2 ? 2 : 3)
     k_cabaret_fused(const Member* __restrict__ mems, const int* __restrict__ prefix, int nmem,

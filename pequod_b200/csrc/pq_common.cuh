@@ -170,15 +170,9 @@ __device__ __forceinline__ bool cab_average_gate(const Member& Mb) {
     return Mb.psi_av != nullptr && Mb.sc->model_time + 0.5 * Mb.sc->dt > Mb.av_threshold;
 }
 
-// Tridiagonal solve geometry: W warps of row chunks per wavenumber column,
-// 8 / W columns per CTA of 256 threads (chosen so a lane's chunk stays
-// short, and its column segments 32 bytes wide: measured on B200 against W
-// one step up and down at 129..2049 rows; at 2049 rows W = 4 would read
-// 16-byte segments, half a DRAM sector).
-__host__ __device__ inline int tri_warps(int jj) {
-    const int Mr = jj - 2;
-    return Mr > 64 ? 2 : 1;
-}
+// Tridiagonal solve geometry: a CTA of 256 threads solves 8 / W wavenumber
+// columns of one mode, each split into 32 W chunks of rows.
+__host__ __device__ inline int tri_warps(int jj) { return jj - 2 > 64 ? 2 : 1; }
 __host__ __device__ inline int tri_ctas(int n, int jj, int L) {
     const int KT = 8 / tri_warps(jj);
     return L * ((n + KT - 1) / KT);
@@ -206,6 +200,17 @@ __device__ __forceinline__ void cta_member(Member& dst, const Member& one, int u
     const unsigned long long* s = reinterpret_cast<const unsigned long long*>(src);
     unsigned long long* d = reinterpret_cast<unsigned long long*>(&dst);
     for (int t = threadIdx.x; t < n; t += blockDim.x) d[t] = s[t];
+}
+
+// Where a kernel reads its descriptor: from its parameters (the field bases
+// then sit in uniform registers, and no CTA waits for a copy) when it is
+// compiled for a context's own launches, else from the shared-memory copy.
+template <bool ONE>
+__device__ __forceinline__ const Member& member_ref(const Member& smem, const Member& param) {
+    if constexpr (ONE)
+        return param;
+    else
+        return smem;
 }
 
 // Map a flat CTA index to (member, local CTA) given prefix sums.

@@ -9,14 +9,14 @@
 //                    CABARET predictor + beta step and the z_to_modes
 //                    projection), scale by 0.5/(ii-1), DST every mode row in
 //                    shared memory, write the spectral rows.
-//   k_tridiag        one CTA per (mode, 8 consecutive wavenumbers): the whole
-//                    column strip is staged in shared memory; each warp owns
-//                    one wavenumber, each lane a chunk of rows, and the
+//   k_tridiag        one CTA per (mode, 4 or 8 consecutive wavenumbers): each lane
+//                    holds a chunk of one column's rows in registers, and the
 //                    forward / backward Thomas recurrences are solved as
 //                    chunked first-order linear recurrences (local sweep,
-//                    warp scan of the affine chunk maps, fix-up sweep).  The
+//                    scan of the affine chunk maps, fix-up sweep).  The
 //                    same CTA accumulates the domain mean of the solution in
-//                    spectral space; the last CTA of a member finishes psiC.
+//                    spectral space (psiC of a closed basin is finished by the
+//                    inverse DST, a channel's by the last CTA).
 //   k_dst (inverse)  one CTA per row j: inverse DST of every mode row, then
 //                    the mass-corrected back-projection (modes_to_z_btcu,
 //                    qg3p_diagnostics.F90:615-635) straight into psi.
@@ -27,6 +27,7 @@
 // and transformed by a radix-4/2 Stockham FFT in shared memory, the real-FFT
 // split gives C_q = R_q + i I_q, and X_2q = -I_q, X_2q+1 = R_0/2 + sum_{p<=q} R_p
 // (the odd outputs are a prefix sum, done as a block scan).
+#include <algorithm>
 #include <type_traits>
 
 #include "pq_common.cuh"
@@ -38,6 +39,12 @@ enum { PRO_PLAIN = 0, PRO_MODAL = 1, PRO_STEP = 2 };
 enum { EPI_SPEC = 0, EPI_HELM = 1, EPI_PV = 2 };
 
 constexpr int TRI_THREADS = 256;
+// CTAs per SM the tridiagonal kernel's registers must allow, by chunk length
+// and storage: 64 registers while they hold a chunk, then 80 (mixed: 1025^2 x 3
+// 142.2 us per step, 145.5 with 128) or 128 (FP64: 174.5, 178.3 with 80, 182 with 64).
+__host__ __device__ constexpr int tri_min_ctas(int RR, bool f32) {
+    return f32 ? (RR <= 8 ? 4 : RR <= 16 ? 3 : 2) : (RR <= 6 ? 4 : RR <= 8 ? 3 : 2);
+}
 
 // ---------------------------------------------------------------------------
 // Row DSTs: one group of P lanes per (row, mode) unit.
@@ -397,7 +404,7 @@ __device__ __forceinline__ void dst_body(const Member* __restrict__ mems, const 
     constexpr bool MX = sizeof(S) == 4;
     __shared__ Member Mb;
     __shared__ double psic_s[PQ_MAXL];                   // closed basin: psiC of the inverse
-    __shared__ double psic_red[dst_max_threads(V) / 32 * PQ_MAXL];
+    __shared__ double psic_red[dst_max_threads(V) / 32 * PQ_MAXL];  // (at least eight warps' room)
     extern __shared__ __align__(16) double sm[];
     pdl_wait();
     int local;
@@ -598,7 +605,15 @@ __device__ __forceinline__ void dst_body(const Member* __restrict__ mems, const 
         }
         // psic_here: this thread's first partial means, in flight with the rows.
         const int KT = 8 / tri_warps(jj), tpm = (n + KT - 1) / KT;
+        // psiC's sum runs on psic_here "threads" (this CTA's, or 256 of which
+        // each warp stands for several warps): the first terms, in flight
+        // with the rows.
         double acc[PQ_MAXL];
+        auto part = [&](int mm, int vt) {
+            double t = 0.0;
+            for (int q = vt; q < tpm; q += psic_here) t += __ldcg(Mb.partials + (long long)mm * tpm + q);
+            return t;
+        };
         if (EPI == EPI_PV && psic_here) {
 #pragma unroll
             for (int mm = 0; mm < PQ_MAXL; ++mm)
@@ -626,22 +641,27 @@ __device__ __forceinline__ void dst_body(const Member* __restrict__ mems, const 
             // CTA (one pass for all modes); the member's
             // first CTA publishes it and flags a NaN (the reference aborts,
             // :504-510) or a value above 1e100 (it warns, :511-517).
-            for (int q = threadIdx.x + nthr; q < tpm; q += nthr)
+            for (int vw = warp; vw < psic_here / 32; vw += nwarp)
 #pragma unroll
-                for (int mm = 0; mm < PQ_MAXL; ++mm)
-                    if (mm < L) acc[mm] += __ldcg(Mb.partials + (long long)mm * tpm + q);
-#pragma unroll
-            for (int mm = 0; mm < PQ_MAXL; ++mm) {
-                if (mm < L) {
-                    const double w = warp_sum(acc[mm]);
-                    if (lane == 0) psic_red[warp * PQ_MAXL + mm] = w;
+                for (int mm = 0; mm < PQ_MAXL; ++mm) {
+                    if (mm < L) {
+                        double t;
+                        if (vw == warp) {
+                            t = acc[mm];
+                            for (int q = threadIdx.x + psic_here; q < tpm; q += psic_here)
+                                t += __ldcg(Mb.partials + (long long)mm * tpm + q);
+                        } else {
+                            t = part(mm, 32 * vw + lane);
+                        }
+                        t = warp_sum(t);
+                        if (lane == 0) psic_red[vw * PQ_MAXL + mm] = t;
+                    }
                 }
-            }
             __syncthreads();
             if (threadIdx.x < L) {
                 const int mm = threadIdx.x;
                 double t = 0.0;
-                for (int w = 0; w < nwarp; ++w) t += psic_red[w * PQ_MAXL + mm];
+                for (int w = 0; w < psic_here / 32; ++w) t += psic_red[w * PQ_MAXL + mm];
                 const double pc = t * Mb.mean_scale;
                 psic_s[mm] = pc;
                 if (local == 0) {
@@ -832,427 +852,356 @@ __host__ __device__ constexpr int dst_min_ctas() {
 }
 
 // ---------------------------------------------------------------------------
-// Tridiagonal solves along j for 8 wavenumbers of one mode.
+// Tridiagonal solves along j for KT = 8 / W wavenumbers of one mode (W warps
+// per column, tri_warps).
 //
-// The strip (Mr = jj - 2 rows x 8 wavenumbers) is staged in shared memory by
-// wavenumber, and within a wavenumber by chunk: row p (0-based) of chunk
-// q = p / R, t = p % R lives at c*CS + q*RS + t with RS = R | 1 odd and CS
-// from tri_cs, so the 32 lanes of a warp (one chunk each) and the half-warps
-// of the staging and write-back phases hit distinct banks.  Lane q of warp c
-// runs the forward and backward Thomas recurrences of its chunk of
-// wavenumber c, on registers for chunks of 4, 8 or 16 rows (RR).
-// Column stride of the strip in doubles: NQ*RS plus a pad that makes the 16
-// threads of a half-warp of the staging and write-back phases -- KT columns
-// x 16/KT chunks each -- hit 16 distinct 8-byte bank pairs: NQ*RS is a
-// multiple of 16, so c*CS + q*RS = RS*(c*16/KT + q) (mod 16) with RS odd.
-// In the solve phase a warp's lanes (one column, 32 chunks) are RS apart.
-__host__ __device__ inline int tri_cs(int NQ, int RS, int KT) { return NQ * RS + (RS * (16 / KT)) % 16; }
+// A lane owns one column's chunk of R <= RR consecutive rows, in registers from
+// its loads to its stores (FULL: R = RR): lane = KT * (chunk in the warp) + column,
+// the 32 W chunks of a column over the CTA's warps.  So a warp's access to row
+// t of its chunks is 32 / KT segments of KT values (32-byte sectors in FP64,
+// KT = 4) -- the transpose needs no shared memory.  The forward and backward
+// Thomas recurrences run as first-order affine recurrences: a local sweep, a
+// scan of the column's affine chunk maps (handed over in shared memory, one chunk per lane
+// of W warps), and a fix-up sweep.  Rows past the column's end are padding of
+// value and pivot 0.  The CTA also accumulates the domain mean of the solution
+// in spectral space.
+//
+// Pivots: explicit up to len (few rows except for the smallest wavenumbers),
+// then the fixed point; a warp beyond len takes the fixed point without a load,
+// the others read theirs from shared memory (loaded beside the rows).
+//
+// What bounds it: the latency of the chain, load to store, in one to three
+// waves.  Against the strip staged in shared memory by cp.async (126 registers
+// and two CTAs per SM at 1025 nodes, shared-memory sweeps unless a chunk had 4,
+// 8 or 16 rows), us per step: 2049^2 x 5 1125 -> 1091 FP64, 842 -> 794 mixed;
+// 1025 x 769 x 3 153 -> 145.5, 1025^2 x 3 178.6 -> 174.5 FP64, 143.3 -> 142.2 mixed;
+// 513 x 385 x 3 55.0 -> 53.7.  The chunks, their scan's order and the sums are that
+// kernel's, so the results are too, bit for bit; chunks spread over more warps and scanned
+// in the warp that holds them measured 2 % faster in the mixed form and lose that.
+//
+// S = float: the mixed form, whose baroclinic spectral rows are FP32 (solved in
+// FP64); the barotropic mode (m = 0) comes from spec64.
+constexpr int TRI_GS_ROWS = 64;  // largest chunk whose columns' pivots fit shared memory (4 x 4096 rows)
+// Doubles between two columns' pivots in shared memory (g(0) .. g(rows)): one
+// of padding per 16, and 16 / KT modulo 16, so that the 16 / KT chunks of KT
+// columns that a half-warp reads hit 16 bank pairs (16-row chunks).
+__host__ __device__ inline int tri_pitch(int rows, int KT) { return (rows + (rows >> 4) + 16) / 16 * 16 + 16 / KT; }
 
-struct PivotRow {
-    const double* piv;  // explicit reciprocal pivots, piv[p - 1] for p <= len
-    int len;
-    double fix;         // the fixed point for p > len
-    __device__ __forceinline__ double operator()(int p) const { return p <= len ? __ldg(&piv[p - 1]) : fix; }
-};
-
-// S = float: the mixed form, whose baroclinic spectral rows are FP32 (staged
-// and solved in FP64); the barotropic mode (m = 0) comes from spec64.
-// Tridiagonal solves along j.  A CTA of 256 threads solves KT = 8 / W
-// wavenumber columns of one mode, W warps per column: the column's rows are
-// split into 32 W chunks of R rows, one per lane, staged in shared memory
-// (chunk q of column c at c*CS + q*RS, RS = R | 1 odd, so a warp's 32 chunk
-// accesses hit 32 banks).  Each lane runs the forward and backward Thomas
-// recurrences of its chunk as first-order affine recurrences (local sweep,
-// scan of the affine chunk maps -- in the warp, then across the column's
-// warps through shared memory -- and a fix-up sweep).  GS = true: the
-// reciprocal pivots of the strip are staged beside it (same layout), so the
-// recurrences never wait on a global load; used whenever both strips fit.
-// The CTA also accumulates the domain mean of the solution in spectral space;
-// the last CTA of a member finishes psiC.
-template <typename S, bool GS, int RR>
-__global__ void __launch_bounds__(TRI_THREADS) k_tridiag(const Member* __restrict__ mems,
-                                                          const int* __restrict__ prefix, int nmem, int do_mean,
-                                                          const __grid_constant__ Member one, int use_one) {
-    __shared__ Member Mb;
-    __shared__ double wpart[TRI_THREADS / 32];
-    __shared__ double wpart2[TRI_THREADS / 32];  // channel: the second wall
-    __shared__ double tot[2][TRI_THREADS / 32][2];  // per-warp affine totals (forward, backward)
+template <typename S, int RR, int KT, bool FULL, bool ONE>
+__global__ void __launch_bounds__(TRI_THREADS, tri_min_ctas(RR, sizeof(S) == 4)) k_tridiag(const Member* __restrict__ mems, const int* __restrict__ prefix,
+                                                  int nmem, int do_mean, const __grid_constant__ Member one,
+                                                  int use_one) {
+    constexpr int W = 8 / KT, NQ = 32 * W;  // warps that scan a column's chunk maps, chunks of a column
+    __shared__ Member Mb_s;
+    __shared__ double maps[2][KT][NQ + 1];  // the chunks' affine maps (A, c); their carries in [0]
+    __shared__ double tot[2][8][2];         // per scanning warp: affine totals (forward, backward)
+    __shared__ double wpart[8], wpart2[8];
+    __shared__ double ends[2][KT];          // channel: the solution's first and last open row
     __shared__ int is_last;
-    extern __shared__ __align__(16) double strip[];
+    extern __shared__ __align__(16) double pivs[];  // [KT][tri_pitch]
     pdl_wait();
-    int local;
-    cta_member(Mb, one, use_one, mems, prefix, nmem, blockIdx.x, &local);
-    __syncthreads();
+    int local = blockIdx.x;
+    if constexpr (!ONE) {
+        cta_member(Mb_s, one, use_one, mems, prefix, nmem, blockIdx.x, &local);
+        __syncthreads();
+    }
+    const Member& Mb = member_ref<ONE>(Mb_s, one);
     const int n = Mb.n, jj = Mb.jj, pitch = Mb.pitch;
-    const int W = tri_warps(jj), KT = 8 / W, NQ = 32 * W;
     const int tiles_per_mode = (n + KT - 1) / KT;
-    const int m = local / tiles_per_mode;
-    const int tile = local - m * tiles_per_mode;
-    const int k0 = tile * KT;  // 0-based column (wavenumber k0+1)
-    const int Mr = jj - 2;
-    const int R = (Mr + NQ - 1) / NQ;
-    const int RS = R | 1;
-    const int CS = tri_cs(NQ, RS, KT);
-    const bool f32 = sizeof(S) == 4 && m > 0;  // this mode's rows are FP32
-    double* spec = ((sizeof(S) == 4) ? Mb.spec64 : reinterpret_cast<double*>(Mb.spec)) + (long long)m * Mb.lstride;
-    float* specf = reinterpret_cast<float*>(Mb.spec) + (long long)m * Mb.lstride;
-    double* gstrip = strip + KT * CS;  // pivots (GS)
-
-    // Stage: thread -> (column c = tid % KT, chunk q = tid / KT); loop over t.
-    // Asynchronous 8-byte copies (cp.async), so the loads of a thread do not
-    // wait for one another; columns past n are zero-filled (source size 0).
-    // FP32 rows are loaded and widened in registers.
-    {
-        const int c = threadIdx.x % KT, q = threadIdx.x / KT;
-        const bool colok = (k0 + c < n);
-        const long long go = (long long)(q * R + 1) * pitch + (colok ? k0 + c : 0);
-        double* sdst = strip + c * CS + q * RS;
-        const int Rq = min(R, Mr - q * R);
-        if (GS) {
-            // g(p) for the rows p = q*R + 1 .. of this chunk: the stored
-            // reciprocal pivots up to len, then the fixed point.
-            double* gdst = gstrip + c * CS + q * RS;
-            if (colok) {
-                const int mk = m * n + k0 + c;
-                const int off = __ldg(&Mb.piv_off[mk]), len = __ldg(&Mb.piv_len[mk]);
-                const double fix = __ldg(&Mb.piv_fix[mk]);
-                const unsigned gbase = (unsigned)__cvta_generic_to_shared(gdst);
-                for (int t = 0; t < Rq; ++t) {
-                    const int pp = q * R + 1 + t;
-                    if (pp <= len)
-                        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(gbase + 8u * t),
-                                     "l"(Mb.piv + off + pp - 1)
-                                     : "memory");
-                    else
-                        gdst[t] = fix;
-                }
-            } else {
-                for (int t = 0; t < Rq; ++t) gdst[t] = 0.0;
-            }
-        }
-        if (!f32) {
-            const double* g = spec + go;
-            const unsigned sbase = (unsigned)__cvta_generic_to_shared(sdst);
-            const int nbytes = colok ? 8 : 0;
-            for (int t = 0; t < Rq; ++t)
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(sbase + 8u * t),
-                             "l"(g + (long long)t * pitch), "r"(nbytes)
-                             : "memory");
-        } else {
-            // FP32 rows: asynchronous 4-byte copies into the upper half of
-            // the chunk's slots (float t at float offset RS + t), widened in
-            // place below (double t covers floats 2t, 2t + 1 < RS + t for
-            // t < RS, so each float is read before it is overwritten).
-            const float* g = specf + go;
-            const unsigned fbase = (unsigned)__cvta_generic_to_shared(reinterpret_cast<float*>(sdst) + RS);
-            const int nbytes = colok ? 4 : 0;
-            for (int t = 0; t < Rq; ++t)
-                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(fbase + 4u * t),
-                             "l"(g + (long long)t * pitch), "r"(nbytes)
-                             : "memory");
-        }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-        if (f32) {
-            const float* fsrc = reinterpret_cast<const float*>(sdst) + RS;
-            for (int t = 0; t < Rq; ++t) sdst[t] = (double)fsrc[t];
-        }
-        // Register sweeps: the rows past the column's end are zeros (after
-        // the widening above, whose staging area they overlap).
-        if (RR > 0 && R == RR)
-            for (int t = max(Rq, 0); t < R; ++t) sdst[t] = 0.0;
-    }
-    __syncthreads();
-
+    const int m = local / tiles_per_mode, tile = local - m * tiles_per_mode;
+    const int Mr = jj - 2, R = FULL ? RR : (Mr + NQ - 1) / NQ;  // rows of a chunk, at most RR
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int c = warp % KT, h = warp / KT;  // column, and which W-th of it
-    const int q = h * 32 + lane;             // chunk
-    const int kk = k0 + c;                   // 0-based wavenumber index
+    const int c = lane & (KT - 1), q = warp * (32 / KT) + lane / KT;  // column and chunk
+    const int kk = tile * KT + c;                                     // 0-based wavenumber index
     const bool active = kk < n;
-    const int a = q * R + 1;                 // first row position (1-based) of the chunk
-    const int cnt = max(0, min(R, Mr - q * R));
-    const int b = a + cnt - 1;
-    double* s = strip + c * CS + q * RS;     // s[t] is position a + t
-    const double* gs = gstrip + c * CS + q * RS;  // GS: gs[t] = g(a + t)
-    PivotRow g{nullptr, 0, 0.0};
-    if (!GS && active) {
-        const int mk = m * n + kk;
-        g = PivotRow{Mb.piv + __ldg(&Mb.piv_off[mk]), __ldg(&Mb.piv_len[mk]), __ldg(&Mb.piv_fix[mk])};
-    }
-    // g(p) for p in [a - 1, b]: g(a - 1) is the previous chunk's last pivot.
-    auto G = [&](int p) -> double {
-        if constexpr (GS) {
-            const int t = p - a;
-            return t >= 0 ? gs[t] : gstrip[c * CS + (q - 1) * RS + (R - 1)];
-        } else {
-            return g(p);
-        }
+    const int a = q * R + 1, b = a + R - 1;  // the chunk's row positions (1-based)
+    const bool f32 = sizeof(S) == 4 && m > 0;  // this mode's rows are FP32
+    // Column kk of this mode's spectral field (row j at sp + j pitch), FP32 or FP64.
+    char* const sp = f32 ? reinterpret_cast<char*>(reinterpret_cast<float*>(Mb.spec) + (long long)m * Mb.lstride + (active ? kk : 0))
+                         : reinterpret_cast<char*>(((sizeof(S) == 4) ? Mb.spec64 : reinterpret_cast<double*>(Mb.spec)) +
+                                                   (long long)m * Mb.lstride + (active ? kk : 0));
+    auto ld = [&](int row) -> double {
+        return f32 ? (double)reinterpret_cast<const float*>(sp)[(long long)row * pitch]
+                   : reinterpret_cast<const double*>(sp)[(long long)row * pitch];
     };
-    // Register sweeps (RR > 0 and R == RR: every chunk exactly RR rows, the
-    // column's end padded with rows whose value and pivot are 0) take the
-    // chunk into v[] and its pivots into gv[] (gv[u] = g(a + u - 1)) once,
-    // without the lambda, so that both arrays stay in registers: the loops
-    // below have constant trip counts and no guards (a guard on a chunk's row
-    // count turns a loop bound into a runtime one and the arrays into local
-    // memory).  A padded row's x is 0 (pivot 0), so it changes no real row,
-    // no chunk map that a real row uses, and no column sum.  Four sweeps on
-    // registers: two shared-memory accesses per row instead of eight.
-    const bool regs = RR > 0 && R == RR;
-    constexpr int RV = RR > 0 ? RR : 1;
-    double v[RV] = {}, gv[RV + 1] = {};
-    if constexpr (RR > 0) {
-        if (regs) {
-#pragma unroll
-            for (int u = 0; u <= RR; ++u) {
-                const int p = a + u - 1;
-                double gg;
-                if constexpr (GS)
-                    gg = u >= 1 ? gs[u - 1] : gstrip[c * CS + max(q - 1, 0) * RS + (R - 1)];
-                else
-                    gg = g(max(p, 1));
-                gv[u] = (active && p >= 1 && p <= Mr) ? gg : 0.0;
-            }
-#pragma unroll
-            for (int t = 0; t < RR; ++t) v[t] = s[t];
-        }
+    // Pivot table entries first: the explicit pivots depend on them.
+    int len = 0, off = 0;
+    double fix = 0.0, wm = 0.0;
+    if (active) {
+        const int mk = m * n + kk;
+        off = __ldg(&Mb.piv_off[mk]);
+        len = __ldg(&Mb.piv_len[mk]);
+        fix = __ldg(&Mb.piv_fix[mk]);
     }
+    // The scanning warp's column weight of the mean, in flight with the rows.
+    if (do_mean && tile * KT + warp % KT < n)
+        wm = __ldg((Mb.periodic ? Mb.wwall : Mb.wmean) + tile * KT + warp % KT);
+    double v[RR];
+    if (f32) {
+        float w[RR];
+#pragma unroll
+        for (int t = 0; t < RR; ++t)
+            w[t] = (active && t < R && a + t <= Mr) ? reinterpret_cast<const float*>(sp)[(long long)(a + t) * pitch] : 0.f;
+#pragma unroll
+        for (int t = 0; t < RR; ++t) v[t] = (double)w[t];
+    } else {
+#pragma unroll
+        for (int t = 0; t < RR; ++t)
+            v[t] = (active && t < R && a + t <= Mr) ? reinterpret_cast<const double*>(sp)[(long long)(a + t) * pitch] : 0.0;
+    }
+    // g(p) at gs[p + p / 16] (0 outside the column), for the warps that read
+    // it: those that start at or before the longest explicit table, and from
+    // the warp that holds the column's end on.
+    len = min(len, Mr);
+    double* const gs = pivs + c * tri_pitch(NQ * R, KT);
+    const double* const piv = Mb.piv + off;
+    if constexpr (RR <= TRI_GS_ROWS) {
+        const int WR = 32 / KT * R;  // rows of a warp
+        const int most = __reduce_max_sync(0xffffffffu, len), e0 = min(Mr, (most / WR + 1) * WR);
+        for (int p = threadIdx.x / KT; p <= e0; p += TRI_THREADS / KT) {
+            double* d = gs + p + (p >> 4);
+            if (p >= 1 && p <= len)
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(d)),
+                             "l"(piv + p - 1)
+                             : "memory");
+            else
+                *d = p == 0 ? 0.0 : fix;
+        }
+        for (int p = max(e0 + 1, Mr / WR * WR) + threadIdx.x / KT; p <= NQ * R; p += TRI_THREADS / KT)
+            gs[p + (p >> 4)] = p <= Mr ? fix : 0.0;
+        cp_commit_wait_all();
+        __syncthreads();
+    }
+    auto G = [&](int p) -> double {
+        if constexpr (RR <= TRI_GS_ROWS)
+            return gs[p + (p >> 4)];
+        else  // longer columns than shared memory holds pivots for
+            return (p < 1 || p > Mr) ? 0.0 : p <= len ? __ldg(piv + p - 1) : fix;
+    };
+    auto F = [&](int) -> double { return fix; };
+    const bool flat = __all_sync(0xffffffffu, a - 1 > len && b <= Mr);
 
+    // (Roundings written out: every instance gives the same bits.)
     // Forward elimination, local: y~_a = f_a, y~_p = f_p - g_{p-1} y~_{p-1};
     // y_p = y~_p + A_p y_{a-1}, A_a = -g_{a-1}, A_p = -g_{p-1} A_{p-1}.
-    double A = 1.0, cend = 0.0;
-    if (active && cnt > 0) {
-        if (regs) {
-            A = (a > 1) ? -gv[0] : 0.0;
-            double y = v[0];
+    double A, y;
+    auto forward = [&](auto g) {
+        A = -g(a - 1);
+        y = v[0];
 #pragma unroll
-            for (int t = 1; t < RV; ++t) {
-                const double gp = gv[t];
-                y = v[t] - gp * y;
+        for (int t = 1; t < RR; ++t) {
+            if (t < R) {
+                const double gp = g(a + t - 1);
+                y = __fma_rn(-gp, y, v[t]);
                 v[t] = y;
-                A = -gp * A;
+                A = __dmul_rn(-gp, A);
             }
-            cend = y;
-        } else {
-            A = (a > 1) ? -G(a - 1) : 0.0;
-            double y = s[0];
-            for (int t = 1; t < cnt; ++t) {
-                const double gp = G(a + t - 1);
-                y = s[t] - gp * y;
-                s[t] = y;
-                A = -gp * A;
-            }
-            cend = y;
         }
-    }
+    };
+    if (flat)
+        forward(F);
+    else
+        forward(G);
+    // Scans run one chunk per lane: warp -> column wc, its half h (of W).
+    const int wc = warp % KT, h = warp / KT, ch = 32 * h + lane;
     // Inclusive scan of the affine chunk maps y_out = c + A y_in in the warp,
     // then the column's earlier warps' totals composed in order.
-    double sA = A, sc = cend;
+    maps[0][c][q] = A;
+    maps[1][c][q] = y;
+    __syncthreads();
+    {
+        double sA = maps[0][wc][ch], sc = maps[1][wc][ch];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const double pA = __shfl_up_sync(0xffffffffu, sA, o);
-        const double pc = __shfl_up_sync(0xffffffffu, sc, o);
-        if (lane >= o) {
-            sc = sc + sA * pc;
-            sA = sA * pA;
+        for (int o = 1; o < 32; o <<= 1) {
+            const double pA = __shfl_up_sync(0xffffffffu, sA, o);
+            const double pc = __shfl_up_sync(0xffffffffu, sc, o);
+            if (lane >= o) {
+                sc = __fma_rn(sA, pc, sc);
+                sA = __dmul_rn(sA, pA);
+            }
         }
-    }
-    if (lane == 31) {
-        tot[0][warp][0] = sA;
-        tot[0][warp][1] = sc;
+        double y0 = 0.0;  // y entering this warp's first chunk
+        if (W > 1) {
+            if (lane == 31) {
+                tot[0][warp][0] = sA;
+                tot[0][warp][1] = sc;
+            }
+            __syncthreads();
+            for (int hh = 0; hh < h; ++hh) y0 = __fma_rn(tot[0][hh * KT + wc][0], y0, tot[0][hh * KT + wc][1]);
+        }
+        const double eA = __shfl_up_sync(0xffffffffu, sA, 1), ec = __shfl_up_sync(0xffffffffu, sc, 1);
+        maps[0][wc][ch] = (lane == 0) ? y0 : __fma_rn(eA, y0, ec);
     }
     __syncthreads();
-    double y0 = 0.0;  // y entering this warp's first chunk
-    for (int hh = 0; hh < h; ++hh) y0 = tot[0][hh * KT + c][1] + tot[0][hh * KT + c][0] * y0;
-    const double eA = __shfl_up_sync(0xffffffffu, sA, 1), ec = __shfl_up_sync(0xffffffffu, sc, 1);
-    const double yin = (lane == 0) ? y0 : ec + eA * y0;
+    const double yin = maps[0][c][q];
     // Fix-up of y, then the local back substitution from the chunk end:
     // x~_b = y_b g_b, x~_p = (y_p - x~_{p+1}) g_p; x_p = x~_p + B_p x_{b+1},
     // B_b = -g_b, B_p = -g_p B_{p+1}.
-    double B = 1.0, cstart = 0.0;
-    if (active && cnt > 0) {
-        if (regs) {
-            double Ap = (a > 1) ? -gv[0] : 0.0;
-            v[0] = v[0] + Ap * yin;
+    double B, x;
+    auto backward = [&](auto g) {
+        double Ap = -g(a - 1);
+        v[0] = __fma_rn(Ap, yin, v[0]);
 #pragma unroll
-            for (int t = 1; t < RV; ++t) {
-                Ap = -gv[t] * Ap;
-                v[t] = v[t] + Ap * yin;
+        for (int t = 1; t < RR; ++t) {
+            if (t < R) {
+                Ap = __dmul_rn(-g(a + t - 1), Ap);
+                v[t] = __fma_rn(Ap, yin, v[t]);
             }
-            const double gb = gv[RV];  // g(b)
-            double x = v[RV - 1] * gb;
-            v[RV - 1] = x;
-            B = -gb;
-#pragma unroll
-            for (int t = RV - 2; t >= 0; --t) {
-                const double gp = gv[t + 1];
-                x = (v[t] - x) * gp;
-                v[t] = x;
-                B = -gp * B;
-            }
-            cstart = x;
-        } else {
-            double Ap = (a > 1) ? -G(a - 1) : 0.0;
-            const double gb = G(b);
-            s[0] = s[0] + Ap * yin;
-            for (int t = 1; t < cnt; ++t) {
-                Ap = -G(a + t - 1) * Ap;
-                s[t] = s[t] + Ap * yin;
-            }
-            double x = s[cnt - 1] * gb;
-            s[cnt - 1] = x;
-            B = -gb;
-            for (int t = cnt - 2; t >= 0; --t) {
-                const double gp = G(a + t);
-                x = (s[t] - x) * gp;
-                s[t] = x;
-                B = -gp * B;
-            }
-            cstart = x;
         }
-    }
+        x = 0.0;
+        B = -1.0;  // B_b = -g_b
+#pragma unroll
+        for (int t = RR - 1; t >= 0; --t) {
+            if (t < R) {
+                const double gp = g(a + t);
+                x = __dmul_rn(__dsub_rn(v[t], x), gp);
+                v[t] = x;
+                B = t == R - 1 ? -gp : __dmul_rn(-gp, B);
+            }
+        }
+    };
+    if (flat)
+        backward(F);
+    else
+        backward(G);
     // Reverse inclusive scan of x_start = c + B x_next, then the column's
     // later warps' totals composed in order.
-    double rB = B, rc = cstart;
+    __syncthreads();  // every lane has read its carry
+    maps[0][c][q] = B;
+    maps[1][c][q] = x;
+    __syncthreads();
+    {
+        double rB = maps[0][wc][ch], rc = maps[1][wc][ch];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const double nB = __shfl_down_sync(0xffffffffu, rB, o);
-        const double nc = __shfl_down_sync(0xffffffffu, rc, o);
-        if (lane + o < 32) {
-            rc = rc + rB * nc;
-            rB = rB * nB;
+        for (int o = 1; o < 32; o <<= 1) {
+            const double nB = __shfl_down_sync(0xffffffffu, rB, o);
+            const double nc = __shfl_down_sync(0xffffffffu, rc, o);
+            if (lane + o < 32) {
+                rc = __fma_rn(rB, nc, rc);
+                rB = __dmul_rn(rB, nB);
+            }
         }
-    }
-    if (lane == 0) {
-        tot[1][warp][0] = rB;
-        tot[1][warp][1] = rc;
+        double x0 = 0.0;  // x entering this warp's last chunk from above
+        if (W > 1) {
+            if (lane == 0) {
+                tot[1][warp][0] = rB;
+                tot[1][warp][1] = rc;
+            }
+            __syncthreads();
+            for (int hh = W - 1; hh > h; --hh) x0 = __fma_rn(tot[1][hh * KT + wc][0], x0, tot[1][hh * KT + wc][1]);
+        }
+        const double nB = __shfl_down_sync(0xffffffffu, rB, 1), nc = __shfl_down_sync(0xffffffffu, rc, 1);
+        maps[0][wc][ch] = (lane == 31) ? x0 : __fma_rn(nB, x0, nc);
     }
     __syncthreads();
-    double x0 = 0.0;  // x entering this warp's last chunk from above
-    for (int hh = W - 1; hh > h; --hh) x0 = tot[1][hh * KT + c][1] + tot[1][hh * KT + c][0] * x0;
-    const double nB = __shfl_down_sync(0xffffffffu, rB, 1), nc = __shfl_down_sync(0xffffffffu, rc, 1);
-    const double xin = (lane == 31) ? x0 : nc + nB * x0;
+    const double xin = maps[0][c][q];
     double lsum = 0.0;
-    if (active && cnt > 0) {
-        if (regs) {
-            double Bp = -gv[RV];
+    auto finish = [&](auto g) {
+        double Bp = -1.0;
 #pragma unroll
-            for (int t = RV - 1; t >= 0; --t) {
-                if (t < RV - 1) Bp = -gv[t + 1] * Bp;
-                const double u = v[t] + Bp * xin;
-                lsum += u;
-                s[t] = u;
-            }
-        } else {
-            double Bp = -G(b);
-            double u = s[cnt - 1] + Bp * xin;
-            s[cnt - 1] = u;
-            lsum += u;
-            for (int t = cnt - 2; t >= 0; --t) {
-                Bp = -G(a + t) * Bp;
-                u = s[t] + Bp * xin;
-                s[t] = u;
-                lsum += u;
+        for (int t = RR - 1; t >= 0; --t) {
+            if (t < R) {
+                const double gp = g(a + t);
+                Bp = t == R - 1 ? -gp : __dmul_rn(-gp, Bp);
+                v[t] = __fma_rn(Bp, xin, v[t]);
+                lsum = __dadd_rn(lsum, v[t]);
             }
         }
-    }
+    };
+    if (flat)
+        finish(F);
+    else
+        finish(G);
     if (Mb.periodic) {
         // periodic_ge (qg3p_helmholtz.F90:565-610): the cyclic closure
         // through the rows 1 and jj, which the Thomas solve above leaves
         // out, as two rank-one corrections with the precomputed b, c.
-        __syncthreads();
-        double z1 = 0.0, zj = 0.0;
+        if (q == 0) ends[0][c] = v[0];                   // row 2 (1-based) after the solve
+#pragma unroll
+        for (int t = 0; t < RR; ++t)
+            if (t < R && a + t == Mr) ends[1][c] = v[t];  // row jj-1
+        double z1i = 0.0, zji = 0.0;  // rows 1 and jj of this mode's spectral field
+        if (active) {
+            z1i = ld(0);
+            zji = ld(jj - 1);
+        }
+        __syncthreads();  // every warp has read rows 1 and jj before they are written
         if (active) {
             const double* pb = Mb.pb + (long long)m * jj * n + kk;
             const double* pc = Mb.pc + (long long)m * jj * n + kk;
-            if (lane == 0) {
-                const int ql = (Mr - 1) / R, tl = (Mr - 1) - ql * R;
-                const double z2 = strip[c * CS];                 // row 2 (1-based) after the solve
-                const double zl = strip[c * CS + ql * RS + tl];  // row jj-1
-                // rows 1 and jj (0 and jj-1) of this mode's spectral field
-                const double z1i = f32 ? (double)specf[kk] : spec[kk];
-                const double zji = f32 ? (double)specf[(long long)(jj - 1) * pitch + kk]
-                                       : spec[(long long)(jj - 1) * pitch + kk];
-                z1 = (z1i - z2) / __ldg(&pb[0]);
-                zj = ((zji - zl) - z1 * __ldg(&pb[(long long)(jj - 1) * n])) / __ldg(&pc[(long long)(jj - 1) * n]);
+            const double z1 = (z1i - ends[0][c]) / __ldg(&pb[0]);
+            const double zj = ((zji - ends[1][c]) - z1 * __ldg(&pb[(long long)(jj - 1) * n])) /
+                              __ldg(&pc[(long long)(jj - 1) * n]);
+            lsum = 0.0;  // the column sum over every row of the closed solution
+#pragma unroll
+            for (int t = 0; t < RR; ++t) {
+                if (t < R && a + t <= Mr) {
+                    const long long row = a + t;  // 0-based grid row
+                    v[t] = (v[t] - z1 * __ldg(&pb[row * n])) - zj * __ldg(&pc[row * n]);
+                    lsum += v[t];
+                }
             }
-            z1 = __shfl_sync(0xffffffffu, z1, 0);
-            zj = __shfl_sync(0xffffffffu, zj, 0);
-        }
-        __syncthreads();  // every warp has read rows 1 and jj before they are written
-        if (active && h == 0 && lane == 0) {
-            const double r0 = z1 - zj * __ldg(&Mb.pc[(long long)m * jj * n + kk]);
-            if (f32) {
-                specf[kk] = (float)r0;
-                specf[(long long)(jj - 1) * pitch + kk] = (float)zj;
-            } else {
-                spec[kk] = r0;
-                spec[(long long)(jj - 1) * pitch + kk] = zj;
+            if (q == 0) {
+                const double r0 = z1 - zj * __ldg(&pc[0]);
+                if (f32) {
+                    reinterpret_cast<float*>(sp)[0] = (float)r0;
+                    reinterpret_cast<float*>(sp)[(long long)(jj - 1) * pitch] = (float)zj;
+                } else {
+                    reinterpret_cast<double*>(sp)[0] = r0;
+                    reinterpret_cast<double*>(sp)[(long long)(jj - 1) * pitch] = zj;
+                }
+                lsum += r0 + zj;
             }
-        }
-        if (active)
-            for (int t = 0; t < cnt; ++t) {
-                const long long row = a + t;  // 0-based grid row
-                s[t] = (s[t] - z1 * __ldg(&Mb.pb[((long long)m * jj + row) * n + kk])) -
-                       zj * __ldg(&Mb.pc[((long long)m * jj + row) * n + kk]);
-            }
-        if (do_mean) {
-            // The column sum over every row of the closed solution.
-            lsum = 0.0;
-            for (int t = 0; t < cnt; ++t) lsum += s[t];
-            if (active && h == 0 && lane == 0) lsum += (z1 - zj * __ldg(&Mb.pc[(long long)m * jj * n + kk])) + zj;
         }
     }
+    if (active) {
+        if (!f32) {
+            double* p = reinterpret_cast<double*>(sp) + (long long)a * pitch;
+#pragma unroll
+            for (int t = 0; t < RR; ++t)
+                if (t < R && a + t <= Mr) p[(long long)t * pitch] = v[t];
+        } else {
+            float* p = reinterpret_cast<float*>(sp) + (long long)a * pitch;
+#pragma unroll
+            for (int t = 0; t < RR; ++t)
+                if (t < R && a + t <= Mr) p[(long long)t * pitch] = (float)v[t];
+        }
+    }
+    pdl_release();
+    if (!do_mean) return;
     // Closed basin: the domain mean of the mode (wmean weights).  Channel:
     // the mean PV of the two walls (zeta_boundary of the solved mode,
     // qg3p_aux.F90:289-379), linear in the column sums: sum_j phi(i, j) =
     // 2 sum_k sin(i k pi / N) C_k, so wall i = 0 gets wwall[k] C_k and wall
     // ii - 1 gets (-1)^(k+1) wwall[k] C_k.
-    double colsum = 0.0, colsum2 = 0.0;
-    if (active && do_mean) {
-        const double cs = warp_sum(lsum);
-        if (Mb.periodic) {
-            const double w = __ldg(&Mb.wwall[kk]);
-            colsum = cs * w;
-            colsum2 = (kk & 1) ? -colsum : colsum;
-        } else {
-            colsum = cs * __ldg(&Mb.wmean[kk]);
-        }
-    }
-    if (lane == 0) {
-        wpart[warp] = colsum;
-        wpart2[warp] = colsum2;
-    }
-    pdl_release();
+    maps[1][c][q] = lsum;  // (its last readers passed a barrier)
     __syncthreads();
     {
-        const int cc = threadIdx.x % KT, qq = threadIdx.x / KT;
-        if (k0 + cc < n) {
-            const long long go = (long long)(qq * R + 1) * pitch + k0 + cc;
-            const double* ssrc = strip + cc * CS + qq * RS;
-            const int Rq = min(R, Mr - qq * R);
-            if (!f32) {
-                double* gdst = spec + go;
-                for (int t = 0; t < Rq; ++t) gdst[(long long)t * pitch] = ssrc[t];
-            } else {
-                float* gdst = specf + go;
-                for (int t = 0; t < Rq; ++t) gdst[(long long)t * pitch] = (float)ssrc[t];
+        const double cs = warp_sum(maps[1][wc][ch]);
+        if (lane == 0) {
+            double t = 0.0, t2 = 0.0;
+            if (tile * KT + wc < n) {
+                t = cs * wm;
+                t2 = (wc & 1) ? -t : t;  // the tile's first column is even
             }
+            wpart[warp] = t;
+            wpart2[warp] = t2;
         }
     }
-    if (!do_mean) return;
+    __syncthreads();
     if (threadIdx.x == 0) {
         double t = 0.0, t2 = 0.0;
-        for (int w = 0; w < TRI_THREADS / 32; ++w) {
+        for (int w = 0; w < 8; ++w) {
             t += wpart[w];
             t2 += wpart2[w];
         }
         Mb.partials[local] = t;
         if (Mb.periodic) Mb.partials[Mb.ntiles_tri + local] = t2;
     }
-    // do_mean 2 (closed basin, an inverse DST of one wave): its CTAs sum the
-    // partials themselves (psiC_m, while their rows load), so no CTA here
-    // waits on a counter.
-    if (!Mb.periodic && do_mean == 2) return;
+    // A closed basin's inverse DST sums the partials itself (psiC_m, while its
+    // rows load), so that no CTA here waits on a counter (1025^2 x 3: 137.9 ->
+    // 135.4 us per step mixed, 180.5 -> 178.2 FP64).
+    if (!Mb.periodic) return;
     if (threadIdx.x == 0) {
         __threadfence();
         const unsigned prev = atomicAdd(&Mb.counters[0], 1u);
@@ -1260,41 +1209,26 @@ __global__ void __launch_bounds__(TRI_THREADS) k_tridiag(const Member* __restric
     }
     __syncthreads();
     if (!is_last) return;
-    // Last CTA of this member, every sum in a fixed order so that the result
-    // is independent of CTA timing.  Closed basin: psiC_m = (sum of partials)
-    // / (g_ii_int g_jj_int).  Channel (modes_to_z_correct_momentum,
+    // Last CTA of this channel, every sum in a fixed order so that the result
+    // is independent of CTA timing (modes_to_z_correct_momentum,
     // qg3p_aux.F90:524-575): the baroclinic modes' coefficients of the two
     // correction functions, inv_corr_a times the wall PV means; the
     // barotropic mode is not corrected.
     __threadfence();
     for (int mm = 0; mm < Mb.L; ++mm) {
         const double t = block_sum_l2(Mb.partials + (long long)mm * tiles_per_mode, tiles_per_mode, 1, wpart);
-        double t2 = 0.0;
-        if (Mb.periodic)
-            t2 = block_sum_l2(Mb.partials + Mb.ntiles_tri + (long long)mm * tiles_per_mode, tiles_per_mode, 1,
-                              wpart2);
+        const double t2 =
+            block_sum_l2(Mb.partials + Mb.ntiles_tri + (long long)mm * tiles_per_mode, tiles_per_mode, 1, wpart2);
         if (threadIdx.x == 0) {
-            double pc, pc2 = 0.0;
-            if (Mb.periodic) {
-                const double* A = Mb.inv_corr_a + 4 * mm;
-                pc = mm == 0 ? 0.0 : A[0] * t + A[2] * t2;
-                pc2 = mm == 0 ? 0.0 : A[1] * t + A[3] * t2;
-                Mb.sc->psiC2[mm] = pc2;
-            } else {
-                pc = t * Mb.mean_scale;
-            }
+            const double* M2 = Mb.inv_corr_a + 4 * mm;
+            const double pc = mm == 0 ? 0.0 : M2[0] * t + M2[2] * t2, pc2 = mm == 0 ? 0.0 : M2[1] * t + M2[3] * t2;
             Mb.sc->psiC[mm] = pc;
+            Mb.sc->psiC2[mm] = pc2;
             if (pc != pc || pc2 != pc2) atomicOr(Mb.status, (int)ST_NAN_PSIC);
             else if (fabs(pc) > 1.0e100 || fabs(pc2) > 1.0e100) atomicOr(Mb.status, (int)ST_LARGE_PSIC);
         }
     }
     if (threadIdx.x == 0) Mb.counters[0] = 0u;
-}
-
-__host__ __device__ inline size_t tri_smem_bytes(int jj) {
-    const int W = tri_warps(jj), KT = 8 / W, NQ = 32 * W;
-    const int Mr = jj - 2, R = (Mr + NQ - 1) / NQ, RS = R | 1;
-    return (size_t)KT * (NQ * RS + 16) * sizeof(double);  // tri_cs pads by at most 15
 }
 
 // ---------------------------------------------------------------------------
@@ -1309,15 +1243,6 @@ int dst_lanes_batched(int M) {
 }
 int dst_max_threads_host(int V) { return dst_max_threads(V); }
 int dst_rows_per_cta_host(int P, int c) { return dst_rows_per_cta(P, c); }
-
-// Whether the inverse DST sums the closed basin's psiC itself: when its grid
-// is one wave (at most four CTAs per SM; measured: +1 % per step at 513^2 x 3,
-// +2.4 % at 129^2, but -1.2 % at 1025^2, whose inverse runs in several waves),
-// so that the tridiagonal kernel's CTAs skip the last-CTA counter.  The
-// tridiagonal launch and the inverse launch decide from the same LaunchSet.
-static int psic_in_inverse(const LaunchSet& ls) {
-    return (!ls.periodic && ls.ctas_dst[1] <= 4 * ls.sm_count) ? 1 : 0;
-}
 
 template <typename S, int V, int PC, int PRO, int EPI>
 static cudaError_t launch_dst_v(const LaunchSet& ls, cudaStream_t st) {
@@ -1346,7 +1271,7 @@ static cudaError_t launch_dst_v(const LaunchSet& ls, cudaStream_t st) {
     const int dir = (EPI == EPI_SPEC) ? 0 : 1;
     return launch_step_kernel(ls.pdl, kern, dim3(ls.ctas_dst[dir]), dim3(threads), bytes, st,
                               ls.members, ls.prefix_dst[dir], ls.nmem, (EPI == EPI_SPEC && !ls.periodic) ? 1 : 0,
-                              ls.dst_group, corr_smem, (EPI == EPI_PV) ? psic_in_inverse(ls) : 0, member_arg(ls),
+                              ls.dst_group, corr_smem, (EPI == EPI_PV && !ls.periodic) ? (ls.ctas_dst[1] <= 4 * ls.sm_count ? threads : 256) : 0, member_arg(ls),
                               member_arg_used(ls), sizeof(S) == 4 ? ls.gemm_bc : 0);
 }
 
@@ -1400,78 +1325,44 @@ cudaError_t launch_dst_inverse(const LaunchSet& ls, int epilogue, int f32, cudaS
     return f32 ? launch_dst<float, PRO_PLAIN, EPI_PV>(ls, st) : launch_dst<double, PRO_PLAIN, EPI_PV>(ls, st);
 }
 
-template <typename S, bool GS, int RR>
-static cudaError_t launch_tri(const LaunchSet& ls, int do_mean, size_t bytes, cudaStream_t st) {
-    cudaError_t e =
-        cudaFuncSetAttribute(k_tridiag<S, GS, RR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+template <typename S, int RR, int KT>
+static cudaError_t launch_tri(const LaunchSet& ls, int do_mean, cudaStream_t st) {
+    constexpr int NQ = 256 / KT;
+    const int R = (ls.maxJ - 2 + NQ - 1) / NQ;
+    const size_t bytes = RR <= TRI_GS_ROWS ? (size_t)KT * tri_pitch(NQ * R, KT) * sizeof(double) : 0;
+    void (*kern)(const Member*, const int*, int, int, Member, int);
+    if (R == RR)
+        kern = member_arg_used(ls) ? k_tridiag<S, RR, KT, true, true> : k_tridiag<S, RR, KT, true, false>;
+    else
+        kern = member_arg_used(ls) ? k_tridiag<S, RR, KT, false, true> : k_tridiag<S, RR, KT, false, false>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return e;
-    cudaError_t le = launch_step_kernel(ls.pdl, k_tridiag<S, GS, RR>, dim3(ls.ctas_tri), dim3(TRI_THREADS), bytes, st,
-                                        ls.members, ls.prefix_tri, ls.nmem, do_mean, member_arg(ls),
-                                        member_arg_used(ls));
-    if (le != cudaSuccess) return le;
-    return cudaGetLastError();
+    return launch_step_kernel(ls.pdl, kern, dim3(ls.ctas_tri), dim3(TRI_THREADS), bytes, st, ls.members,
+                              ls.prefix_tri, ls.nmem, do_mean, member_arg(ls), member_arg_used(ls));
 }
 
-// Resident CTAs per SM of k_tridiag<S, GS, RR> with `bytes` of shared memory
-// (cached per host thread for the last size asked: contexts may be driven
-// from several threads).
-template <typename S, bool GS, int RR>
-static int tri_resident(size_t bytes) {
-    thread_local size_t cached_bytes = 0;
-    thread_local int cached = 0;
-    if (cached_bytes != bytes) {
-        int n = 0;
-        if (cudaFuncSetAttribute(k_tridiag<S, GS, RR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) !=
-                cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_tridiag<S, GS, RR>, TRI_THREADS, bytes) !=
-                cudaSuccess) {
-            cudaGetLastError();
-            n = 0;
-        }
-        cached_bytes = bytes;
-        cached = n;
-    }
-    return cached;
-}
-
-// Register sweeps read each pivot once per row, from the pivot table: staging
-// the pivots beside the strip measured slower for them (1025^2 x 3: 33.4 us
-// without, 36.5 with, mixed; 31.8 / 35.2 FP64), so only the shared-memory
-// sweeps stage them.
-template <typename S, int RR>
-static cudaError_t launch_tri_gs(const LaunchSet& ls, int do_mean, size_t bytes, size_t gs_limit, cudaStream_t st) {
-    if constexpr (RR > 0) {
-        return launch_tri<S, false, RR>(ls, do_mean, bytes, st);
-    } else {
-        const bool gs =
-            2 * bytes <= gs_limit && tri_resident<S, true, RR>(2 * bytes) >= tri_resident<S, false, RR>(bytes);
-        return gs ? launch_tri<S, true, RR>(ls, do_mean, 2 * bytes, st)
-                  : launch_tri<S, false, RR>(ls, do_mean, bytes, st);
-    }
-}
-
-cudaError_t launch_tridiag(const LaunchSet& ls, int do_mean_in, int f32, cudaStream_t st) {
-    const size_t bytes = tri_smem_bytes(ls.maxJ);
-    const int do_mean = (do_mean_in && psic_in_inverse(ls)) ? 2 : do_mean_in;
-    // Pivots staged beside the strip when both fit (the FP32 form, whose
-    // strip is loaded synchronously, only while two CTAs still fit an SM) and
-    // the staging costs no resident CTA per SM: measured on B200, staging that
-    // lowers occupancy is slower (1025 x 1025 x 3: -2 % FP64, -4 % mixed per
-    // step; 2049 x 2049 x 5 FP64: -4 %).
-    // Chunks of 4, 8 or 16 rows are solved in registers (the instance for
-    // the largest member's chunk length; a member whose chunks differ takes
-    // the shared-memory sweeps inside it).
+// The instance that holds chunks of R rows (every member of a launch has
+// ls.maxJ rows per column); beyond 32 rows they spill.
+template <typename S>
+static cudaError_t launch_tri_rows(const LaunchSet& ls, int do_mean, cudaStream_t st) {
     const int W = tri_warps(ls.maxJ), R = (ls.maxJ - 2 + 32 * W - 1) / (32 * W);
-    if (f32) {
-        if (R == 4) return launch_tri_gs<float, 4>(ls, do_mean, bytes, 100 * 1024, st);
-        if (R == 8) return launch_tri_gs<float, 8>(ls, do_mean, bytes, 100 * 1024, st);
-        if (R == 16) return launch_tri_gs<float, 16>(ls, do_mean, bytes, 100 * 1024, st);
-        return launch_tri_gs<float, 0>(ls, do_mean, bytes, 100 * 1024, st);
-    }
-    if (R == 4) return launch_tri_gs<double, 4>(ls, do_mean, bytes, 160 * 1024, st);
-    if (R == 8) return launch_tri_gs<double, 8>(ls, do_mean, bytes, 160 * 1024, st);
-    if (R == 16) return launch_tri_gs<double, 16>(ls, do_mean, bytes, 160 * 1024, st);
-    return launch_tri_gs<double, 0>(ls, do_mean, bytes, 160 * 1024, st);
+    if (W == 1) return launch_tri<S, 2, 8>(ls, do_mean, st);
+    if (R <= 3) return launch_tri<S, 3, 4>(ls, do_mean, st);
+    if (R <= 4) return launch_tri<S, 4, 4>(ls, do_mean, st);
+    if (R <= 6) return launch_tri<S, 6, 4>(ls, do_mean, st);
+    if (R <= 8) return launch_tri<S, 8, 4>(ls, do_mean, st);
+    if (R <= 12) return launch_tri<S, 12, 4>(ls, do_mean, st);
+    if (R <= 16) return launch_tri<S, 16, 4>(ls, do_mean, st);
+    if (R <= 20) return launch_tri<S, 20, 4>(ls, do_mean, st);
+    if (R <= 24) return launch_tri<S, 24, 4>(ls, do_mean, st);
+    if (R <= 32) return launch_tri<S, 32, 4>(ls, do_mean, st);
+    if (R <= 64) return launch_tri<S, 64, 4>(ls, do_mean, st);
+    if (R <= 128) return launch_tri<S, 128, 4>(ls, do_mean, st);
+    return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_tridiag(const LaunchSet& ls, int do_mean, int f32, cudaStream_t st) {
+    return f32 ? launch_tri_rows<float>(ls, do_mean, st) : launch_tri_rows<double>(ls, do_mean, st);
 }
 
 }  // namespace pq
