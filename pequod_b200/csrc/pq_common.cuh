@@ -114,7 +114,9 @@ struct Member {
     void* rel;
     double* psi_other;  // leapfrog: the other time level's psi and rel
     void* rel_other;
-    void* helm_io;    // in/out buffer of the stand-alone helm() entry point
+    void* helm_io;    // in/out buffer of the stand-alone helm() entry point (a field, or the caller's
+    int io_pitch;     //   dense device array), with its row pitch and
+    long long io_ls;  //   layer stride in doubles
     void* flux_i;
     void* flux_j;
     void* spec;

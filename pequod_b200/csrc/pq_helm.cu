@@ -454,8 +454,8 @@ __device__ __forceinline__ void dst_body(const Member* __restrict__ mems, const 
         };
         if constexpr (PRO == PRO_PLAIN) {
             // The stand-alone helm input (helm_io) is FP64 in either form.
-            const double* src = reinterpret_cast<const double*>(Mb.helm_io) + um * ls +
-                                (long long)(ju < jend ? ju : jend - 1) * pitch;
+            const double* src = reinterpret_cast<const double*>(Mb.helm_io) + um * Mb.io_ls +
+                                (long long)(ju < jend ? ju : jend - 1) * Mb.io_pitch;
             if (fp64_mode(um)) {
                 stage_unit<V>(ubuf(um, ur), p, P, N, Mb.was, [&](int k) { return cff * __ldg(src + k); });
             } else if (gemm_bc) {
@@ -709,7 +709,7 @@ __device__ __forceinline__ void dst_body(const Member* __restrict__ mems, const 
         // i = ii zeroed (:758-761); ge_local zeroes psi(2:ii-1, 1)
         // (:1055-1057).  helm_io is FP64 in either form (the mixed form's
         // FP32 units are widened).
-        double* io = reinterpret_cast<double*>(Mb.helm_io) + um * ls + (long long)ju * pitch;
+        double* io = reinterpret_cast<double*>(Mb.helm_io) + um * Mb.io_ls + (long long)ju * Mb.io_pitch;
         if (interior) {
             if (fp64_mode(um)) {
                 const double* buf = ubuf(um, ur);
