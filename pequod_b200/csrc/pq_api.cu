@@ -83,6 +83,28 @@ PivotTables build_pivots(int ii, int jj, int L, const double* ss) {
 }
 
 // Copy between a dense (ii, jj, L) host/device array and a pitched field.
+bool kernel_can_address(const double* p, size_t n, int device) {
+    using Fn = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+    static const Fn query = [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &fn, cudaEnableDefault, &q) != cudaSuccess) fn = nullptr;
+        return reinterpret_cast<Fn>(fn);
+    }();
+    if (!query || (size_t)p % sizeof(double)) return false;
+    CUpointer_attribute what[5] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_ORDINAL,
+                                   CU_POINTER_ATTRIBUTE_IS_MANAGED, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                   CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    unsigned type = 0, managed = 0;
+    int ord = -1;
+    CUdeviceptr base = 0;
+    size_t size = 0;
+    void* out[5] = {&type, &ord, &managed, &base, &size};
+    const CUdeviceptr a = (CUdeviceptr)(size_t)p;
+    return query(5, what, out, a) == CUDA_SUCCESS && type == CU_MEMORYTYPE_DEVICE && !managed && ord == device &&
+           base && a >= base && a - base <= size && n * sizeof(double) <= size - (a - base);
+}
+
 int copy_in(pq_ctx* c, void* dst, const double* src, int kind) {
     const size_t w = (size_t)c->ii * sizeof(double);
     CK(cudaMemcpy2DAsync(dst, (size_t)c->pitch * sizeof(double), src, w, w, (size_t)c->jj * c->L,
@@ -867,7 +889,7 @@ int pq_helm(pq_ctx* c, double* zeta, int ptr_kind) {
     if (!c || !zeta) return PQ_ERR_ARG;
     CK(cudaSetDevice(c->device));
     c->last_launches = 3;
-    if (ptr_kind == PQ_PTR_DEVICE) {
+    if (ptr_kind == PQ_PTR_DEVICE && kernel_can_address(zeta, (size_t)c->ii * c->jj * c->L, c->device)) {
         // No copies in and out of the context (65 x 65: 50.2 -> 42.8 us per call).
         const int rc = run_helm(c, c->cur, PRO_PLAIN, EPI_HELM, 0, zeta);
         if (rc) return rc;

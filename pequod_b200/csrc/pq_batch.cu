@@ -22,6 +22,7 @@
 #include <cstring>
 #include <map>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "pq_ctx.h"
@@ -158,6 +159,25 @@ int enqueue_solve(pq_batch* b) {
     if (!rc) rc = phase(b->tri_cls, 1);
     if (!rc) rc = phase(b->dst_cls, 2);
     return rc;
+}
+
+// Every member's array can be addressed by the copy kernel and overlaps no
+// other: members' copies are not ordered within a launch.
+bool separate_arrays(const pq_batch* b, double* const* zeta) try {
+    std::vector<std::pair<size_t, size_t>> at;
+    at.reserve(b->mem.size());
+    for (size_t k = 0; k < b->mem.size(); ++k) {
+        const pq_ctx* c = b->mem[k];
+        const size_t n = (size_t)c->ii * c->jj * c->L;
+        if (!kernel_can_address(zeta[k], n, b->device)) return false;
+        at.emplace_back((size_t)zeta[k], n * sizeof(double));
+    }
+    std::sort(at.begin(), at.end());
+    for (size_t k = 1; k < at.size(); ++k)
+        if (at[k - 1].first + at[k - 1].second > at[k].first) return false;
+    return true;
+} catch (...) {
+    return false;
 }
 
 }  // namespace
@@ -493,11 +513,9 @@ int pq_batch_sync(pq_batch* b) {
 
 int pq_batch_helm(pq_batch* b, double* const* zeta, int ptr_kind) {
     if (!b || !zeta) return PQ_ERR_ARG;
-    if (ptr_kind == PQ_PTR_DEVICE) {
+    if (ptr_kind == PQ_PTR_DEVICE && separate_arrays(b, zeta)) {
         // Two launches of copies in place of two pitched copies per member.
         const int n = (int)b->mem.size();
-        for (int k = 0; k < n; ++k)
-            if (!zeta[k]) return PQ_ERR_ARG;
         BK(cudaSetDevice(b->device));
         auto copy = [&](int in) -> cudaError_t {
             for (int k0 = 0; k0 < n; k0 += kCopyMembers) {

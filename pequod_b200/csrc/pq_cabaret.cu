@@ -713,9 +713,9 @@ __device__ __forceinline__ bool count_done(const Member& Mb, double umax, unsign
 // Persistent: a member's CTAs (at most the resident ones, cabaret_ctas) share
 // its (layer, strip, band) sweeps through a counter (counters[3]); each warp
 // claims the next sweep when it finishes one, so warps run until the queue is
-// empty instead of idling in partly filled CTAs and waves.  The boundary
-// bands (bounds checks and boundary branches: slower) are claimed first, so
-// the last sweeps claimed are interior ones.  The last CTA resets the counter.
+// empty instead of idling in partly filled CTAs and waves.  The sweeps at a
+// wall (slower) are claimed first, so the last sweeps claimed are interior
+// ones.  The last warp of a member resets the counter (finish_step).
 template <bool PRED, typename T, int NC, bool ONE>
 __global__ void __launch_bounds__(CAB_WARPS * 32, NC == 2 ? 2 : 3)
     k_cabaret_fused(const Member* __restrict__ mems, const int* __restrict__ prefix, int nmem,

@@ -5,11 +5,11 @@
 // solve along j with precomputed reciprocal pivots (ge_local, :1028-1059),
 // and the inverse DST (helm, :614-769).  Here that is three kernels:
 //
-//   k_dst (forward)  one CTA per interior row j: load (optionally apply the
+//   k_dst (forward)  a CTA per few interior rows: load (optionally apply the
 //                    CABARET predictor + beta step and the z_to_modes
 //                    projection), scale by 0.5/(ii-1), DST every mode row in
 //                    shared memory, write the spectral rows.
-//   k_tridiag        one CTA per (mode, 4 or 8 consecutive wavenumbers): each lane
+//   k_tridiag        a CTA per (mode, KT consecutive wavenumbers): each lane
 //                    holds a chunk of one column's rows in registers, and the
 //                    forward / backward Thomas recurrences are solved as
 //                    chunked first-order linear recurrences (local sweep,
@@ -17,14 +17,14 @@
 //                    same CTA accumulates the domain mean of the solution in
 //                    spectral space (psiC of a closed basin is finished by the
 //                    inverse DST, a channel's by the last CTA).
-//   k_dst (inverse)  one CTA per row j: inverse DST of every mode row, then
+//   k_dst (inverse)  a CTA per few rows: inverse DST of every mode row, then
 //                    the mass-corrected back-projection (modes_to_z_btcu,
 //                    qg3p_diagnostics.F90:615-635) straight into psi.
 //
 // DST-I of length n = N - 1 (N = ii - 1 = 2^p), FFTPACK convention
 // X_k = 2 sum_m x_m sin(m k pi / N): the sequence is pre-twiddled into a real
 // sequence c of length N (as sint1 does), c is packed into N/2 complex points
-// and transformed by a radix-4/2 Stockham FFT in shared memory, the real-FFT
+// and transformed by a radix-8/4/2 Stockham FFT, the real-FFT
 // split gives C_q = R_q + i I_q, and X_2q = -I_q, X_2q+1 = R_0/2 + sum_{p<=q} R_p
 // (the odd outputs are a prefix sum, done as a block scan).
 #include <algorithm>

@@ -61,3 +61,36 @@ def test_batch_of_device_arrays(n):
     assert pq.lib().pq_batch_helm(b.ctx, ptrs, pq.PTR_DEVICE) == pq.PQ_OK
     assert all(np.array_equal(t.cpu().numpy().transpose(2, 1, 0), w) for t, w in zip(d, want))
     b.close()
+
+
+@pytest.mark.parametrize("where", ["misaligned", "null", "shared"])
+def test_arrays_the_kernels_do_not_address(where):
+    """Arrays that take the copies instead: the same results, the same refusals."""
+    import torch
+
+    shapes = [(17, 9, 1), (17, 9, 1)]
+    b = pq.Batch(shapes, [np.array([0.1]), np.array([0.1])])
+    rng = np.random.default_rng(5)
+    rhs = [np.asfortranarray(rng.standard_normal(s)) for s in shapes]
+    want = b.helm(rhs)
+    n = 17 * 9
+    host = np.concatenate([r.transpose(2, 1, 0).ravel() for r in rhs])
+    raw = torch.zeros(16 * n + 8, dtype=torch.uint8, device="cuda")
+    off = 4 if where == "misaligned" else 0
+    raw[off : off + 16 * n] = torch.from_numpy(host.view(np.uint8)).cuda()
+    torch.cuda.synchronize()
+    second = 0 if where == "shared" else 8 * n
+    at = [raw.data_ptr() + off, raw.data_ptr() + off + second]
+    if where == "null":  # refused
+        at[1] = None
+    ptrs = (C.POINTER(C.c_double) * 2)(*[C.cast(C.c_void_p(a), C.POINTER(C.c_double)) for a in at])
+    rc = pq.lib().pq_batch_helm(b.ctx, ptrs, pq.PTR_DEVICE)
+    if at[1] is None:
+        assert rc != pq.PQ_OK
+    else:
+        assert rc == pq.PQ_OK
+        got = np.frombuffer(raw.cpu().numpy()[off : off + 16 * n].tobytes(), dtype=np.float64)
+        assert np.array_equal(got[:n].reshape(1, 9, 17).transpose(2, 1, 0), want[0])
+        if where == "misaligned":
+            assert np.array_equal(got[n:].reshape(1, 9, 17).transpose(2, 1, 0), want[1])
+    b.close()
