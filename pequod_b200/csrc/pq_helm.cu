@@ -603,7 +603,6 @@ __device__ __forceinline__ void dst_body(const Member* __restrict__ mems, const 
                 for (int q = lane; q < cw; q += 32) cp16(d + 2 * q, g + 2 * q, ok);
             }
         }
-        // psic_here: this thread's first partial means, in flight with the rows.
         const int KT = 8 / tri_warps(jj), tpm = (n + KT - 1) / KT;
         // psiC's sum runs on psic_here "threads" (this CTA's, or 256 of which
         // each warp stands for several warps): the first terms, in flight
@@ -1244,6 +1243,7 @@ int dst_lanes_batched(int M) {
 int dst_max_threads_host(int V) { return dst_max_threads(V); }
 int dst_rows_per_cta_host(int P, int c) { return dst_rows_per_cta(P, c); }
 
+constexpr int PSIC_CTAS = 592;
 template <typename S, int V, int PC, int PRO, int EPI>
 static cudaError_t launch_dst_v(const LaunchSet& ls, cudaStream_t st) {
     const int M = ls.maxN / 2, L = ls.maxL;
@@ -1254,6 +1254,13 @@ static cudaError_t launch_dst_v(const LaunchSet& ls, cudaStream_t st) {
     // corr rows in shared memory only while four CTAs still fit an SM
     const int corr_smem = (EPI == EPI_PV && !ls.periodic && bytes + cbytes <= 56 * 1024) ? 1 : 0;
     if (corr_smem) bytes += cbytes;
+    // The number of strided sums psiC is taken in: a CTA's threads (one pass), or
+    // 256 when a member has more than PSIC_CTAS CTAs of rows.  Either order is
+    // the one such a problem has always had; which one it is depends on the
+    // member's own rows alone, so that a run merged with others, on any device,
+    // adds as it does alone (every member of a launch has ls.maxJ rows).
+    const int psic_here =
+        (EPI == EPI_PV && !ls.periodic) ? ((ls.maxJ + R - 1) / R <= PSIC_CTAS ? threads : 256) : 0;
     // The inverse with 64-lane units of 8 values takes the register-capped
     // instance (1025^2 x 3: 41.1 -> 37.3 us mixed, 44.5 -> 41.7 us FP64).
     void (*kern)(const Member*, const int*, int, int, int, int, int, Member, int, int);
@@ -1271,8 +1278,8 @@ static cudaError_t launch_dst_v(const LaunchSet& ls, cudaStream_t st) {
     const int dir = (EPI == EPI_SPEC) ? 0 : 1;
     return launch_step_kernel(ls.pdl, kern, dim3(ls.ctas_dst[dir]), dim3(threads), bytes, st,
                               ls.members, ls.prefix_dst[dir], ls.nmem, (EPI == EPI_SPEC && !ls.periodic) ? 1 : 0,
-                              ls.dst_group, corr_smem, (EPI == EPI_PV && !ls.periodic) ? (ls.ctas_dst[1] <= 4 * ls.sm_count ? threads : 256) : 0, member_arg(ls),
-                              member_arg_used(ls), sizeof(S) == 4 ? ls.gemm_bc : 0);
+                              ls.dst_group, corr_smem, psic_here, member_arg(ls), member_arg_used(ls),
+                              sizeof(S) == 4 ? ls.gemm_bc : 0);
 }
 
 // The compile-time geometries: what the defaults select (dst_lanes_default
