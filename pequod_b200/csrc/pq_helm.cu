@@ -457,11 +457,11 @@ __device__ __forceinline__ void dst_body(const Member* __restrict__ mems, const 
             const double* src = reinterpret_cast<const double*>(Mb.helm_io) + um * Mb.io_ls +
                                 (long long)(ju < jend ? ju : jend - 1) * Mb.io_pitch;
             if (fp64_mode(um)) {
-                stage_unit<V>(ubuf(um, ur), p, P, N, Mb.was, [&](int k) { return cff * __ldg(src + k); });
+                stage_unit<V>(ubuf(um, ur), p, P, N, Mb.was, [&](int k) { return cff * __ldcg(src + k); });
             } else if (gemm_bc) {
-                for (int t = p; t < M; t += P) put(um, ur, t, cff * __ldg(src + (t ? t : M)), cff * __ldg(src + N - t - (t ? 0 : M)));
+                for (int t = p; t < M; t += P) put(um, ur, t, cff * __ldcg(src + (t ? t : M)), cff * __ldcg(src + N - t - (t ? 0 : M)));
             } else {
-                stage_unit<V>(ubuf32(um, ur), p, P, N, Mb.was_f, [&](int k) { return (float)(cff * __ldg(src + k)); });
+                stage_unit<V>(ubuf32(um, ur), p, P, N, Mb.was_f, [&](int k) { return (float)(cff * __ldcg(src + k)); });
             }
         } else {
             const double dt = Mb.sc->dt, ta = Mb.sc->tweight_a;
@@ -563,8 +563,8 @@ __device__ __forceinline__ void dst_body(const Member* __restrict__ mems, const 
 #pragma unroll
                                 for (int l = 0; l < LC; ++l) {
                                     const bool in = has(l) && t < M;
-                                    va[q][l] = in ? __ldg(row + l * ls + k) : (S)0;
-                                    vb[q][l] = in ? __ldg(row + l * ls + N - k) : (S)0;
+                                    va[q][l] = in ? __ldcg(row + l * ls + k) : (S)0;
+                                    vb[q][l] = in ? __ldcg(row + l * ls + N - k) : (S)0;
                                 }
                             }
 #pragma unroll
@@ -622,16 +622,16 @@ __device__ __forceinline__ void dst_body(const Member* __restrict__ mems, const 
         const long long ro = um * ls + (long long)(interior ? ju : 1) * pitch - 1;
         if (fp64_mode(um)) {
             const double* g = (MX ? Mb.spec64 : reinterpret_cast<const double*>(Mb.spec)) + ro;
-            stage_unit<V>(ubuf(um, ur), p, P, N, Mb.was, [&](int k) { return interior ? __ldg(g + k) : 0.0; });
+            stage_unit<V>(ubuf(um, ur), p, P, N, Mb.was, [&](int k) { return interior ? __ldcg(g + k) : 0.0; });
         } else if (gemm_bc) {
             // Rows the tensor-core DST already took back to node values:
             // straight to the positions the back-projection reads.
             const float* g = reinterpret_cast<const float*>(Mb.gbuf) + ro;
             float* d = ubuf32(um, ur);
-            for (int k = 1 + p; k <= n; k += P) d[xpad(k)] = interior ? __ldg(g + k) : 0.f;
+            for (int k = 1 + p; k <= n; k += P) d[xpad(k)] = interior ? __ldcg(g + k) : 0.f;
         } else {
             const float* g = reinterpret_cast<const float*>(Mb.spec) + ro;
-            stage_unit<V>(ubuf32(um, ur), p, P, N, Mb.was_f, [&](int k) { return interior ? __ldg(g + k) : 0.f; });
+            stage_unit<V>(ubuf32(um, ur), p, P, N, Mb.was_f, [&](int k) { return interior ? __ldcg(g + k) : 0.f; });
         }
         if (EPI == EPI_PV && psic_here) {
             // psiC_m = (sum of the tridiagonal CTAs' partial means of mode m)
