@@ -427,7 +427,7 @@ int pq::create_ctx(pq_ctx** out, const pq_model_desc* d, int device, bool helm_o
                                              : cabaret_ctas(ii, jj, L, cab_sh, cab_kernel, mixed);
 
     // Tables: exp(-2 pi i t / M) and exp(-2 pi i t / N), laid out the way the
-    // row DST reads them (pq_helm.cu: three pass plans, five lane widths).
+    // row DST reads them (pq_dst.cuh: three pass plans, five lane widths).
     std::vector<double2> tw0(M), ws0(M), tw((size_t)3 * M), wsplit((size_t)5 * M);
     for (int t = 0; t < M; ++t) {
         const long double a = 2.0L * 3.141592653589793238462643383279502884L * (long double)t / (long double)M;

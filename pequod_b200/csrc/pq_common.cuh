@@ -74,7 +74,7 @@ struct Member {
     double htot;
     double mean_scale;  // 1 / (g_ii_int * g_jj_int)
     // Helmholtz tables (shared between members of the same size)
-    const double2* tw;      // [3][M] pass twiddles, by pass plan (pq_helm.cu)
+    const double2* tw;      // [3][M] pass twiddles, by pass plan (pq_dst.cuh)
     const double* was;      // [N/2] 2 sin(k pi / N), index k (0 unused)
     const double2* wsplit;  // [5][M] exp(-2 pi i q / N), by values per lane
     const double* wmean;    // [n]  2 * sum_i sin(i k pi / N), index k-1
@@ -164,6 +164,17 @@ struct Member {
 // CTAs overlap only this grid's tail.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 __device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+
+// Asynchronous copies to shared memory: 16 bytes (zeros unless ok), and the wait
+// for all of the thread's copies.
+__device__ __forceinline__ void cp16(void* dst, const void* src, bool ok) {
+    const unsigned sa = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sa), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void cp_commit_wait_all() {
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+    asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+}
 
 // Whether the CABARET step now running accumulates the time average (model
 // time after the step's first half increment, qg3.F90:656, 672).  Read by

@@ -1,0 +1,10 @@
+// pq_dst_plain.cu -- The forward row DST of the stand-alone solves.
+#include "pq_dst.cuh"
+
+namespace pq {
+
+cudaError_t launch_dst_plain(const LaunchSet& ls, int f32, cudaStream_t st) {
+    return f32 ? launch_dst<float, PRO_PLAIN, EPI_SPEC>(ls, st) : launch_dst<double, PRO_PLAIN, EPI_SPEC>(ls, st);
+}
+
+}  // namespace pq

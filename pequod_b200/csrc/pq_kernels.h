@@ -62,7 +62,7 @@ inline cudaError_t launch_step_kernel(int pdl, void (*kernel)(KArgs...), dim3 gr
 }
 
 
-// pq_helm.cu
+// pq_helm.cu, pq_dst_*.cu, pq_tridiag.cu
 // Lanes per DST unit for complex length M = N/2 and L modes by default
 // (dir 0 forward, 1 inverse), and rows per DST CTA for P lanes per unit and
 // row-group setting c.
