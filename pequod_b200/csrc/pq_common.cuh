@@ -184,8 +184,9 @@ __device__ __forceinline__ bool cab_average_gate(const Member& Mb) {
 }
 
 // Tridiagonal solve geometry: a CTA of 256 threads solves 8 / W wavenumber
-// columns of one mode, each split into 32 W chunks of rows.
-__host__ __device__ inline int tri_warps(int jj) { return jj - 2 > 64 ? 2 : 1; }
+// columns of one mode, each split into 32 W chunks of rows (four columns of
+// more than 7104 rows would not fit shared memory, two do).
+__host__ __device__ inline int tri_warps(int jj) { return jj - 2 > 7104 ? 4 : jj - 2 > 64 ? 2 : 1; }
 __host__ __device__ inline int tri_ctas(int n, int jj, int L) {
     const int KT = 8 / tri_warps(jj);
     return L * ((n + KT - 1) / KT);
