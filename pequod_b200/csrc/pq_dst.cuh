@@ -173,6 +173,15 @@ __device__ __forceinline__ void put_pair(T* buf, int t, int N, T xa, T xb, const
     else
         buf[0] = (T)0;
 }
+// One node of the pair (odd: node N - t) by itself, given the other's value.
+template <typename T>
+__device__ __forceinline__ void put_node(T* buf, int t, bool odd, int N, T own, T other, const T* __restrict__ was) {
+    const int k = t ? t : N >> 1;
+    if (odd && !t)
+        buf[0] = (T)0;
+    else
+        buf[cidx(odd ? N - t : k)] = mad(__ldg(&was[k]), own + other, own - other);
+}
 // A unit's own row, straight from global memory (fetch(k) is x_k): V pairs per lane,
 // at most eight of them in flight.
 template <int V, typename T, typename F>
@@ -410,6 +419,17 @@ __device__ __forceinline__ void dst_body(const Member* __restrict__ mems, const 
                 put_pair(ubuf32(m, r), t, N, (float)xa, (float)xb, Mb.was_f);
             }
         };
+        // The same of one node (odd: N - t), given the other's value.
+        [[maybe_unused]] auto put1 = [&](int m, int r, int t, bool odd, double own, double other) {
+            if (fp64_mode(m)) {
+                put_node(ubuf(m, r), t, odd, N, own, other, Mb.was);
+            } else if (gemm_bc) {
+                if (j0 + r < jend && (t || !odd))
+                    reinterpret_cast<float*>(Mb.gbuf)[m * ls + (long long)(j0 + r) * pitch - 1 + (odd ? N - t : t ? t : N >> 1)] = (float)own;
+            } else {
+                put_node(ubuf32(m, r), t, odd, N, (float)own, (float)other, Mb.was_f);
+            }
+        };
         if constexpr (PRO == PRO_PLAIN) {
             // The stand-alone helm input (helm_io) is FP64 in either form.
             const double* src = reinterpret_cast<const double*>(Mb.helm_io) + um * Mb.io_ls +
@@ -453,7 +473,7 @@ __device__ __forceinline__ void dst_body(const Member* __restrict__ mems, const 
                 // arithmetic and the stores of res_beta and zeta.
                 auto step_node = [&](int j, int k, bool ok, double (&z)[LC]) {
                     const long long o = (long long)j * pitch + k;
-                    double a0[LC], a1[LC], a2[LC], a3[LC], a4[LC];
+                    S a0[LC], a1[LC], a2[LC], a3[LC], a4[LC];  // (widened at their use: no load waits)
 #pragma unroll
                     for (int l = 0; l < LC; ++l) {
                         if (has(l) && ok) {
@@ -470,9 +490,9 @@ __device__ __forceinline__ void dst_body(const Member* __restrict__ mems, const 
                         double zz = 0.0;
                         if (has(l) && ok) {
                             const long long ol = o + l * ls;
-                            zz = a0[l] + 0.5 * dt * a1[l];
-                            const double rbn = dt * (0.5 * (a3[l] + a2[l]) * Mb.beta[l]);
-                            zz = zz + (1.0 + ta) * rbn - ta * a4[l];
+                            zz = (double)a0[l] + 0.5 * dt * (double)a1[l];
+                            const double rbn = dt * (0.5 * ((double)a3[l] + (double)a2[l]) * Mb.beta[l]);
+                            zz = zz + (1.0 + ta) * rbn - ta * (double)a4[l];
                             rb[ol] = (S)rbn;
                             zp[ol] = (S)zz;
                             if (MX) zz = (double)(S)zz;  // the stored (FP32) value
@@ -504,6 +524,31 @@ __device__ __forceinline__ void dst_body(const Member* __restrict__ mems, const 
                 const int G = FLAT && P < 32 ? 32 / P : 1;
                 auto row_of = [&](int r0, int i) { return FLAT ? r0 + (PC ? i / M : i >> Mb.logM) : r0; };
                 auto pair_of = [&](int i) { return FLAT ? i & (M - 1) : i; };
+                if constexpr (PRO == PRO_STEP && !EX && V <= 16) {
+                    // More than five layers: a node per lane, its pair's other
+                    // from the next lane, so that the predictor's loads of
+                    // a node (five per layer) and one projection fit the registers.
+                    // (Whole warps: the shuffle below, also where 2 M < 32.)
+                    for (int r0 = 0; r0 < R; r0 += G) {
+                        for (int t0 = threadIdx.x; t0 < ((2 * G * M + 31) & ~31); t0 += nthr) {
+                            const bool in = t0 < 2 * G * M, odd = t0 & 1;
+                            const int i = in ? t0 >> 1 : 0, r = row_of(r0, i), t = pair_of(i);
+                            const int j = min(j0 + r, jend - 1), k = odd ? N - t : t ? t : M;
+                            double z[LC];
+                            step_node(j, k, in && j0 + r < jend && (t || !odd), z);
+#pragma unroll 1
+                            for (int m = 0; m < L; ++m) {
+                                double sum = 0.0;
+#pragma unroll
+                                for (int l = 0; l < LC; ++l)
+                                    if (has(l)) sum += Mb.z2m[m * PQ_MAXL + l] * z[l];
+                                const double own = cff * sum, next = __shfl_xor_sync(0xffffffffu, own, 1);
+                                if (in) put1(m, r, t, odd, own, t ? next : own);
+                            }
+                        }
+                    }
+                    return;
+                }
                 for (int r0 = 0; r0 < R; r0 += G) {
                     const bool ok0 = j0 + r0 < jend;
                     const int jr0 = ok0 ? j0 + r0 : jend - 1;
@@ -817,7 +862,7 @@ __global__ void __launch_bounds__(dst_max_threads(V), MINB)
 // 8 values.
 template <int V, int PC, int PRO, int EPI>
 __host__ __device__ constexpr int dst_min_ctas() {
-    if (PRO == PRO_STEP) return V <= 8 ? 2 : 0;
+    if (PRO == PRO_STEP) return V <= 8 ? 2 : V == 16 ? 1 : 0;
     if (V == 16) return 2;
     if (EPI == EPI_SPEC && PRO == PRO_MODAL) return V <= 8 ? 3 : 0;
     return (EPI == EPI_PV && V == 8 && PC == 64) ? 3 : 0;
