@@ -878,8 +878,12 @@ static cudaError_t launch_dst_v(const LaunchSet& ls, cudaStream_t st) {
     const int threads = L * R * (M / V);
     size_t bytes = dst_units_len(L, R, ls.maxN, sizeof(S) == 4) * sizeof(double);
     const size_t cbytes = (size_t)R * (L - 1) * ls.maxPitch * sizeof(double);
-    // corr rows in shared memory only while four CTAs still fit an SM
-    const int corr_smem = (EPI == EPI_PV && !ls.periodic && bytes + cbytes <= 56 * 1024) ? 1 : 0;
+    constexpr int MINB = dst_min_ctas<V, PC, PRO, EPI>();
+    // corr rows in shared memory while as many CTAs fit an SM beside them as the
+    // registers allow: four; two of more than 192 threads with 128 registers
+    // (513^2 x 8: 41.4 us without, 40.0 with); one of 32 values (2049 x 257 x 6: 94, 81).
+    const size_t room = (V == 32 ? 200 : (MINB == 0 && threads > 192) ? 100 : 56) * 1024;
+    const int corr_smem = (EPI == EPI_PV && !ls.periodic && bytes + cbytes <= room) ? 1 : 0;
     if (corr_smem) bytes += cbytes;
     // The number of strided sums psiC is taken in: a CTA's threads (one pass), or
     // 256 when a member has more than PSIC_CTAS CTAs of rows.  Either order is
@@ -889,7 +893,6 @@ static cudaError_t launch_dst_v(const LaunchSet& ls, cudaStream_t st) {
     const int psic_here =
         (EPI == EPI_PV && !ls.periodic) ? ((ls.maxJ + R - 1) / R <= PSIC_CTAS ? threads : 256) : 0;
     void (*kern)(const Member*, const int*, int, int, int, int, int, Member, int, int);
-    constexpr int MINB = dst_min_ctas<V, PC, PRO, EPI>();
     if constexpr (MINB > 0)
         kern = k_dst_capped<S, V, PC, PRO, EPI, MINB>;
     else
