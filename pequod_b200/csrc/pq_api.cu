@@ -82,7 +82,6 @@ PivotTables build_pivots(int ii, int jj, int L, const double* ss) {
     return t;
 }
 
-// Copy between a dense (ii, jj, L) host/device array and a pitched field.
 bool kernel_can_address(const double* p, size_t n, int device) {
     using Fn = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
     static const Fn query = [] {
@@ -105,6 +104,7 @@ bool kernel_can_address(const double* p, size_t n, int device) {
            base && a >= base && a - base <= size && n * sizeof(double) <= size - (a - base);
 }
 
+// Copy between a dense (ii, jj, L) host/device array and a pitched field.
 int copy_in(pq_ctx* c, void* dst, const double* src, int kind) {
     const size_t w = (size_t)c->ii * sizeof(double);
     CK(cudaMemcpy2DAsync(dst, (size_t)c->pitch * sizeof(double), src, w, w, (size_t)c->jj * c->L,
@@ -421,7 +421,7 @@ int pq::create_ctx(pq_ctx** out, const pq_model_desc* d, int device, bool helm_o
     const bool mixed = d->precision == PQ_PREC_MIXED;
     const long long nodes = (long long)ii * jj * L;
     const int cab_kernel = helm_only ? 0 : (mixed && jj > 1500) ? 2 : nodes < (mixed ? 280000 : 370000) ? 0 : 1;
-    const int cab_sh = helm_only ? kMinBand : cab_kernel == 2 ? 24 : cabaret_band(ii, jj, L, 1, mixed);
+    const int cab_sh = helm_only ? kMinBand : cab_kernel == 2 ? 24 : cabaret_band(ii, jj, L, mixed);
     const int ntiles_cab = d->periodic_j ? channel_ctas(ii, jj)
                            : cab_kernel == 0 ? cabaret_tile_ctas(ii, jj, L)
                                              : cabaret_ctas(ii, jj, L, cab_sh, cab_kernel, mixed);

@@ -136,9 +136,8 @@ __device__ __forceinline__ double mn(double a, double b) { return a < b ? a : b;
 __device__ __forceinline__ float mx(float a, float b) { return fmaxf(a, b); }
 __device__ __forceinline__ float mn(float a, float b) { return fminf(a, b); }
 // The input rows of an iteration come in 16-byte chunks (cp.async.cg: no line of the L1 cache
-// is held while a copy is in flight; the 8-byte copies of the edge sweep hold
-// three lines each, and the L1 cache left beside the rings bounds how many
-// fly).  The rows of an iteration lie one after another in a ring stage --
+// is held while a copy is in flight; a field's row copied 8 bytes per lane holds
+// three lines, and the L1 cache left beside the rings bounds how many fly).  The rows of an iteration lie one after another in a ring stage --
 // first the FP64 ones, then the T ones -- and instruction q of a class copies
 // chunks 32 q .. 32 q + 31 of them: a lane's chunk belongs to one field for
 // the whole sweep, so its address is one pointer that moves a row down per
@@ -1283,14 +1282,14 @@ static int cabaret_resident(int nc, bool f32) {
 // which every round begun so far holds them all.  At most 40 rows: taller
 // bands measured slower at 2049^2 x 5 (86 rows 661 us, 29 rows 601), where
 // the L2 cache no longer holds a row from one band to the next.
-int cabaret_band(int ii, int jj, int L, int nc, bool f32) {
-    const long long W = (long long)CAB_WARPS * cabaret_resident(nc, f32);
-    const int sw = cab_sw(nc), ns = (ii + sw - 1) / sw;
+int cabaret_band(int ii, int jj, int L, bool f32) {
+    const long long W = (long long)CAB_WARPS * cabaret_resident(1, f32);
+    const int sw = cab_sw(1), ns = (ii + sw - 1) / sw;
     double best = 1e300;
     int band = 4;
     for (int sh = 4; sh <= 40; ++sh) {
         const int nb = (jj + sh - 1) / sh;
-        const int nsi = ii < 32 * nc ? 0 : std::max(0, (ii - 32 * nc) / sw - (4 + sw - 1) / sw + 1);
+        const int nsi = ii < 32 ? 0 : std::max(0, (ii - 32) / sw - (4 + sw - 1) / sw + 1);
         const int nbi = jj < 6 + sh ? 0 : std::max(0, (jj - 6 - sh) / sh - (6 + sh - 1) / sh + 1);
         const long long nI = (long long)nsi * nbi * L, nE = (long long)ns * nb * L - nI;
         const double c = sh + 5, e = 1.5 * c;

@@ -103,12 +103,12 @@ int copy_in_state(pq_ctx* c, void* dst, const double* src, int kind);
 int copy_out_state(pq_ctx* c, double* dst, const void* src, int kind);
 int check_status(pq_ctx* c);
 int upload_members(pq_ctx* c);
-// dense: for PRO_PLAIN / EPI_HELM, a dense (ii, jj, L) device array to solve
-// in place instead of the context's helm_io.
 // True if a kernel on `device` may address the n doubles at p (the device's own
 // memory, all in one allocation, aligned): other arrays are copied, and the
 // copy reports what it cannot read.
 bool kernel_can_address(const double* p, size_t n, int device);
+// dense: for PRO_PLAIN / EPI_HELM, a dense (ii, jj, L) device array to solve
+// in place instead of the context's helm_io.
 int run_helm(pq_ctx* c, int par, int prologue, int epilogue, int mean, double* dense = nullptr);
 // The inversion of a step (forward DST with `prologue`, tridiagonal,
 // inverse DST with the back-projection), through the tensor-core DST when

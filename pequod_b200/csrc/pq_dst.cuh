@@ -41,9 +41,11 @@ template <typename T2> __device__ __forceinline__ T2 c_mi(T2 a) {  // a * (-i)
 }
 
 // The FP32 transform's products and sums are written out as the multiply-adds
-// they are, so that every instance (lanes, values per lane, one member or
-// many) rounds alike whatever the compiler would contract around them: a
-// mixed run's trajectory does not depend on the geometry of its launches.
+// they are, so that every instance of a geometry (its lanes at compile time or
+// not, one member or many) rounds alike whatever the compiler would contract
+// around them: a mixed run is the same alone and merged with others.  (Other
+// lanes per unit round differently: the passes' radices follow the values per
+// lane, and the prefix sum of the odd outputs is grouped by lane.)
 // FP64 leaves the contraction to the compiler, which folds a twiddle product
 // into the butterfly's sums (two operations fewer, one rounding fewer).
 __device__ __forceinline__ double mad(double a, double b, double c) { return fma(a, b, c); }
@@ -361,8 +363,8 @@ __host__ __device__ inline size_t dst_units_len(int L, int R, int N, bool mixed)
 
 // The row-DST kernel's body; k_dst and k_dst_capped below are its kernels.
 //
-// PC > 0: the lanes per unit P at compile time (the default geometries of the
-// grids up to 2049 nodes), hence N, M and the pitch: every index of the
+// PC > 0: the lanes per unit P at compile time (most default geometries,
+// launch_dst), hence N, M and the pitch: every index of the
 // transform is then a lane's base plus an immediate.
 template <typename S, int V, int PC, int PRO, int EPI>
 __device__ __forceinline__ void dst_body(const Member* __restrict__ mems, const int* __restrict__ prefix, int nmem,
@@ -519,15 +521,16 @@ __device__ __forceinline__ void dst_body(const Member* __restrict__ mems, const 
                 };
                 // Two values per lane: the rows of units narrower than a warp (G of
                 // them) side by side, so that their loads are in flight together
-                // (33 x 33 x 3: 12.8 us one row after the other, 10.7).
+                // (33 x 33 x 3 mixed: 12.8 us one row after the other, 10.8).
                 constexpr bool FLAT = V == 2 && PC < 32;
                 const int G = FLAT && P < 32 ? 32 / P : 1;
                 auto row_of = [&](int r0, int i) { return FLAT ? r0 + (PC ? i / M : i >> Mb.logM) : r0; };
                 auto pair_of = [&](int i) { return FLAT ? i & (M - 1) : i; };
                 if constexpr (PRO == PRO_STEP && !EX && V <= 16) {
                     // More than five layers: a node per lane, its pair's other
-                    // from the next lane, so that the predictor's loads of
-                    // a node (five per layer) and one projection fit the registers.
+                    // from the next lane, so that the predictor's loads of a
+                    // node (five per layer) and one projection fit the registers
+                    // (1025^2 x 8, pairs: 235 us FP64 and 280 mixed; 169, 166).
                     // (Whole warps: the shuffle below, also where 2 M < 32.)
                     for (int r0 = 0; r0 < R; r0 += G) {
                         for (int t0 = threadIdx.x; t0 < ((2 * G * M + 31) & ~31); t0 += nthr) {
@@ -856,10 +859,12 @@ __global__ void __launch_bounds__(dst_max_threads(V), MINB)
                  int corr_smem, int psic_here, const __grid_constant__ Member one, int use_one, int gemm_bc) {
     dst_body<S, V, PC, PRO, EPI>(mems, prefix, nmem, row_offset, c, corr_smem, psic_here, one, use_one, gemm_bc);
 }
-// CTAs per SM the registers must allow (0: no bound): the forward DST three
-// of 256 threads up to 8 values per lane; the inverse of 64-lane units of 8
-// values three; 16 values two of 320; the forward with the predictor two up to
-// 8 values.
+// CTAs per SM the registers must allow (0: no bound; the bound's CTAs have 256
+// threads, 320 with 16 values): the forward DST three up to 8 values per lane,
+// the inverse of 64-lane units of 8 values three, 16 values two.  With the predictor
+// two up to 8 values (513^2 x 4 FP64 20.9 us, 27.0 without a bound; 1025^2 x 4 65, 78;
+// the smallest grids lose 2 us at eight layers) and one with 16, which lets its
+// loads take the registers (1025^2 x 5 FP64 98.9 us, 123 without).
 template <int V, int PC, int PRO, int EPI>
 __host__ __device__ constexpr int dst_min_ctas() {
     if (PRO == PRO_STEP) return V <= 8 ? 2 : V == 16 ? 1 : 0;
@@ -881,7 +886,7 @@ static cudaError_t launch_dst_v(const LaunchSet& ls, cudaStream_t st) {
     constexpr int MINB = dst_min_ctas<V, PC, PRO, EPI>();
     // corr rows in shared memory while as many CTAs fit an SM beside them as the
     // registers allow: four; two of more than 192 threads with 128 registers
-    // (513^2 x 8: 41.4 us without, 40.0 with); one of 32 values (2049 x 257 x 6: 94, 81).
+    // (513^2 x 8 FP64: 41.0 us without, 30.9 with); one of 32 values (2049 x 257 x 6: 94, 83).
     const size_t room = (V == 32 ? 200 : (MINB == 0 && threads > 192) ? 100 : 56) * 1024;
     const int corr_smem = (EPI == EPI_PV && !ls.periodic && bytes + cbytes <= room) ? 1 : 0;
     if (corr_smem) bytes += cbytes;
@@ -907,7 +912,9 @@ static cudaError_t launch_dst_v(const LaunchSet& ls, cudaStream_t st) {
 }
 
 // The compile-time geometries: what the defaults select (dst_lanes_default
-// for a step, dst_lanes_batched for the stand-alone solves).
+// for a step, dst_lanes_batched for the stand-alone solves) from 65 (33) to 2049
+// nodes, but for a step of five or more layers at 1025 nodes, of six or more at 2049,
+// and a stand-alone solve at 2049: one-warp units of 16 and 32 values.
 template <typename S, int PRO, int EPI>
 static cudaError_t launch_dst(const LaunchSet& ls, cudaStream_t st) {
     const int P = ls.dst_lanes[EPI == EPI_SPEC ? 0 : 1], V = ls.maxN / 2 / P;

@@ -19,7 +19,7 @@ struct LaunchSet {
     int ctas_rows_interior;
     const int* prefix_rows_all;       // jj CTAs per member
     int ctas_rows_all;
-    const int* prefix_tri;            // L * ceil(n / 8) CTAs per member
+    const int* prefix_tri;            // tri_ctas(n, jj, L) CTAs per member
     int ctas_tri;
     const int* prefix_cab;            // cabaret_ctas(ii, jj, L) CTAs per member
     int ctas_cab;
@@ -87,8 +87,8 @@ cudaError_t launch_quad(const LaunchSet& ls, int f32, int lf, cudaStream_t st);
 // CTAs of the (persistent) sweep kernel per member: band height sh, nc
 // columns per lane, FP32 fields when f32; at most the CTAs resident at once.
 int cabaret_ctas(int ii, int jj, int L, int sh, int nc, bool f32);
-// The default band height of that kernel.
-int cabaret_band(int ii, int jj, int L, int nc, bool f32);
+// The default band height of that kernel with one column per lane.
+int cabaret_band(int ii, int jj, int L, bool f32);
 int cabaret_tile_ctas(int ii, int jj, int L);     // CTAs of the tile kernel per member
 cudaError_t launch_rel(const LaunchSet& ls, int f32, cudaStream_t st);
 cudaError_t launch_init_finish(const LaunchSet& ls, int f32, cudaStream_t st);

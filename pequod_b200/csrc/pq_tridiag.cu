@@ -34,9 +34,10 @@ __host__ __device__ constexpr int tri_min_ctas(int RR, bool f32) {
 // What bounds it: the latency of the chain, load to store, in one to three
 // waves.  Against the strip staged in shared memory by cp.async (126 registers
 // and two CTAs per SM at 1025 nodes, shared-memory sweeps unless a chunk had 4,
-// 8 or 16 rows), us per step: 2049^2 x 5 1125 -> 1091 FP64, 842 -> 794 mixed;
-// 1025 x 769 x 3 153 -> 145.5, 1025^2 x 3 178.6 -> 174.5 FP64, 143.3 -> 142.2 mixed;
-// 513 x 385 x 3 55.0 -> 53.7.  The chunks, their scan's order and the sums are that
+// 8 or 16 rows), us per step: 2049^2 x 5 1125 -> 1093 FP64, 842 -> 793 mixed;
+// 1025 x 769 x 3 153 -> 143, 1025^2 x 3 179 -> 175 FP64, 142.5 -> 140 mixed.  At
+// 25 to 31 rows a chunk the mixed form's kernel is 13 % slower on 2049 columns
+// (2049 x 1540 x 3: 84 -> 94 us) and 20 % faster on 257 (28.5 -> 23.4).  The chunks, their scan's order and the sums are that
 // kernel's, so the results are too, bit for bit; chunks spread over more warps and scanned
 // in the warp that holds them measured 2 % faster in the mixed form and lose that.
 //
